@@ -34,6 +34,7 @@ struct Scalars {
     double abs_floor;   // absolute floor on ||r||^2 (reference abs_div_tol term)
     double tol2;        // relative tolerance squared
     double inner_floor2;// minimum inner relative reduction squared
+    double pass_margin; // share of the goal on ||r||^2 that a pass aims at
     double objective;   // chain objective / misc reductions
     double divmax, div2;// divergence statistics
     float alpha_f, beta_f, sigma, inv_sigma;

@@ -277,6 +277,7 @@ static int build_levels(mhdproj_ctx* ctx) {
     P.m = d[0] * d[1] * d[2];
     CK(dalloc(ctx, &P.ainv, (size_t)P.m * P.m * sizeof(float)));
     P.bottom_img = nullptr;
+    P.w_min_bytes = ctx->pipelined ? 48ll << 20 : 0;
     mg_plan_bottom(P);
     if (P.bottom_from > 0) {
         CK(dalloc(ctx, (char**)&P.bottom_img, (size_t)P.bottom.img_floats * sizeof(float)));
@@ -302,7 +303,17 @@ static int build_levels(mhdproj_ctx* ctx) {
             CK(dalloc(ctx, &P.e0, (size_t)ctx->n * 4));
             const size_t rbytes = P.precision == 0 ? 16 : 8;
             for (int l = 0; l < F; l++) {
-                CK(dalloc(ctx, (char**)&P.lv[l].sm, (size_t)P.lv[l].L.g.n() * rbytes));
+                const Grid3& gl = P.lv[l].L.g;
+                CK(dalloc(ctx, (char**)&P.lv[l].sm,
+                          std::max((size_t)gl.n() * rbytes, P.precision != 0 && tma_level_ok(gl) ? tma_record_bytes(gl) : 0)));
+                if (run_level_ok(P.precision, gl))
+                    P.lv[l].passes = PASS_RUN;
+                else if (P.precision == 0 && pair_level_init(gl, P.lv[l].sm, P.lv[l].e))
+                    P.lv[l].passes = PASS_PAIR;
+                else if (P.precision != 0 && tma_level_init(P.precision, gl, P.lv[l].sm))
+                    P.lv[l].passes = PASS_TMA;
+                else
+                    P.lv[l].passes = PASS_ASYNC;
                 if (l > 0) CK(dalloc(ctx, (char**)&P.lv[l].eo, (size_t)P.lv[l].L.g.n() * vbytes));
                 if (l > 0 && P.w_from > 0 && l >= P.w_from && l <= P.w_to) {
                     CK(dalloc(ctx, (char**)&P.lv[l].r2, (size_t)P.lv[l].L.g.n() * vbytes));
@@ -676,17 +687,16 @@ static uint64_t kernels_pass_start(const mhdproj_ctx* ctx) {
 }
 
 static void enqueue_precondition(mhdproj_ctx* ctx) {
-    if (ctx->use_mg) mg_vcycle(ctx->mg, ctx->stream);
+    if (ctx->pipelined)
+        mg_vcycle_fused(ctx->mg, ctx->r, nullptr, nullptr, false, ctx->partials, ctx->n_active, ctx->stream);
+    else if (ctx->use_mg) mg_vcycle(ctx->mg, ctx->stream);
     else k_jacobi<<<ctx->L.grid, ctx->L.block, 0, ctx->stream>>>(ctx->L.g, ctx->coef, ctx->r, ctx->z, ctx->sc);
 }
 // Pass start of the pipelined CG: z = B r0 and rz (the first search step
 // then takes p = z).
 static void enqueue_pass_start(mhdproj_ctx* ctx) {
-    if (ctx->pipelined) {
-        mg_vcycle_fused(ctx->mg, ctx->r, nullptr, nullptr, false, ctx->partials, ctx->n_active, ctx->stream);
-        return;
-    }
     enqueue_precondition(ctx);
+    if (ctx->pipelined) return;
     Fields F = fields(ctx);
     launch_dot_rz(ctx->L, F, 1, ctx->stream);
 }
@@ -836,12 +846,28 @@ static int solve(mhdproj_ctx* ctx, float* x_hi, float* x_lo, mhdproj_stats* st, 
     return 0;
 }
 
-static void begin_scalars(mhdproj_ctx* ctx) {
+static void begin_scalars(mhdproj_ctx* ctx, bool adjoint = false) {
     const double tol2 = (double)ctx->opt.rel_tol * ctx->opt.rel_tol;
     const double h = ctx->grid.h;
     const double abs_floor = (double)ctx->opt.abs_div_tol * ctx->opt.abs_div_tol * h * h * h * h * (double)ctx->n_active;
     // FP32 CG reduces its own residual by about 1e-5 reliably; refine beyond.
-    launch_init_scalars(ctx->sc, tol2, abs_floor, 1e-10, (int)ctx->opt.max_iterations, ctx->stream);
+    // A pass aims at half the tolerance on ||r||.  Three half-steps of smoothing
+    // leave a smoother residual than two, whose error is larger at the same
+    // norm (cylinder 64^3 at half the tolerance: pressure 1.2e-5 off FP64,
+    // against 3.5e-6 with two), so with them on every level above the bottom
+    // sub-cycle a pass aims at 1/16 (4e-7; about one iteration more), and
+    // where other levels lie between, whose two half-steps leave rougher
+    // residuals, at 1/8.  An adjoint's right-hand side has more weight on
+    // smooth modes, whose error a residual shows least: a quarter of that (vjp
+    // jet 192x160x132: 4e-6 off FP64 at 1/16, 1e-7 at 1/64, 7e-7 with two
+    // half-steps at half the tolerance).
+    const MGPlan& P = ctx->mg;
+    double pass_margin = 1.0 / 4;
+    if (ctx->pipelined && P.lv[0].passes != PASS_PAIR) {
+        pass_margin = P.bottom_from > 0 && P.fused_levels >= P.bottom_from ? 1.0 / 256 : 1.0 / 64;
+        if (adjoint) pass_margin /= 16;
+    }
+    launch_init_scalars(ctx->sc, tol2, abs_floor, 1e-10, pass_margin, (int)ctx->opt.max_iterations, ctx->stream);
 }
 
 static const char* const MEANFREE_ADJOINT =
@@ -1024,7 +1050,7 @@ extern "C" int mhdproj_project_host(mhdproj_ctx* ctx, const float* alpha, const 
 // -------------------------------------------------------------- adjoint
 static int vjp_gb300(mhdproj_ctx* ctx, const float* gu, const float* gv, const float* gw, const float* gp, float dt,
                      float* ou, float* ov, float* ow, mhdproj_stats* st) {
-    begin_scalars(ctx);
+    begin_scalars(ctx, true);
     Fields F = fields(ctx);
     launch_adj_rhs(ctx->L, F, gu, gv, gw, gp, dt, ctx->stream);
     ctx->launches += 2;

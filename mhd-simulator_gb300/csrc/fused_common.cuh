@@ -80,6 +80,15 @@ template <> __device__ __forceinline__ void st2<__nv_bfloat16>(__nv_bfloat16* p,
     *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v.x, v.y);
 }
 
+// Wrapped or absent coordinate along one axis, any number of periods away (a
+// halo or the rest of a tile can be wider than the grid).
+__device__ __forceinline__ int axis_wrap(int c, int n, bool periodic, bool* ok) {
+    *ok = periodic || (c >= 0 && c < n);
+    if (c < 0) return periodic ? n - 1 - (-1 - c) % n : 0;
+    if (c >= n) return periodic ? c % n : n - 1;
+    return c;
+}
+
 // The smoother records in HBM are split along whole grid rows: row (y, z)
 // holds its nx/2 even-x records, then its nx/2 odd-x records.  Position of
 // column x in its row:
@@ -144,6 +153,71 @@ __device__ __forceinline__ float2 divide2(float2 s, float2 d) {
 
 // Red half (x parity of the red cells) of row y at plane z; x0-4 is even.
 __device__ __forceinline__ int red_half(int y, int z) { return (y + z) & 1; }
+
+// A quad's offset in a plane of one colour (rows of HW values) from its split
+// offset (row * RW + 2q).
+__device__ __forceinline__ int half_off(int o) { return o - (o / RW) * HW; }
+
+// Over-relaxation of the black half-step between two red ones.
+constexpr float SOR_BLACK = 1.2f;
+
+// End of a pre-smoothing pass that updated the residual: ||r||^2 over all
+// blocks, counts the iteration and decides convergence (not after a pass that
+// gave up on a copy).  Every thread of every block calls it.
+__device__ __forceinline__ void finish_residual_norm(float rr_thread, Scalars* sc, double* partials, int nblocks,
+                                                     double* sh) {
+    double v1[1] = {(double)rr_thread};
+    block_sum<1>(v1, sh);
+    if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[8])) {
+        double tot[1];
+        finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[8]);
+        if (threadIdx.x + threadIdx.y == 0 && !sc->stalled) {
+            const double rr = tot[0];
+            sc->rr = rr;
+            sc->iterations += 1;
+            sc->total_iterations += 1;
+            if (!isfinite(rr)) {
+                sc->nonfinite = 1;
+                sc->converged = 1;
+            } else if (rr <= sc->rr_target || sc->total_iterations >= sc->max_total) {
+                sc->converged = 1;
+            }
+        }
+    }
+}
+// End of the finest level's post-smoothing pass: r . z over all blocks, the CG
+// step's beta, the next V-cycle's sigma.
+__device__ __forceinline__ void finish_rz(double rz_thread, Scalars* sc, double* partials, int nblocks,
+                                          long long n_active, double* sh) {
+    double v1[1] = {rz_thread};
+    block_sum<1>(v1, sh);
+    if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[9])) {
+        double tot[1];
+        finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[9]);
+        if (threadIdx.x + threadIdx.y == 0 && !sc->stalled) {
+            const double rz = tot[0];
+            if (!isfinite(rz)) {
+                sc->nonfinite = 1;
+                sc->converged = 1;
+            } else if (!(rz > 0.0)) {
+                sc->breakdown = 1;
+                sc->converged = 1;
+            } else if (sc->first) {
+                sc->rz = rz;
+                sc->beta = 0.0;
+                sc->beta_f = 0.0f;
+            } else {
+                sc->beta = rz / sc->rz;
+                sc->beta_f = (float)sc->beta;
+                sc->rz = rz;
+            }
+            // z is in units of this V-cycle's sigma; the next V-cycle
+            // scales by the RMS of the residual it will be given.
+            sc->inv_sigma_z = sc->inv_sigma;
+            set_sigma_from(sc, sc->rr, n_active);
+        }
+    }
+}
 
 template <int N>
 using Phase = std::integral_constant<int, N>;

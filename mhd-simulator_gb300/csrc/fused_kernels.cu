@@ -3,22 +3,28 @@
 //
 // Pre-smoothing pass (k_presmooth_restrict), per level:
 //   [fine level, inside CG] r <- r - alpha q       (the CG residual update)
-//   red half-step from a zero correction            e_red   = sigma r / d
-//   black half-step                                 e_black = (sigma r + sum beta e_red) / d
-//   residual and restriction                        rc      = 1/4 P^T (sigma r - A e)
+//   red half-step from a zero correction            e_red    = sigma r / d
+//   black half-step, over-relaxed (SOR_BLACK)       e_black  = w (sigma r + sum beta e_red) / d
+//   red half-step                                   e_red   += (sum beta e_black) / d
+//   residual and restriction                        rc       = 1/4 P^T (sigma r - A e)
 // Post-smoothing pass (k_prolong_postsmooth), per level:
 //   prolongation                                    e <- e + w P ec
-//   black half-step, then red half-step             z       = the smoothed correction
+//   red, black (over-relaxed), red half-steps       z        = the smoothed correction
 //   [fine level] r . z for the CG step length.
-// Both march a 64 x 16 (x, y) tile along z.  The stages of one pass run as a
-// pipeline over planes: the pre-smoothing pass forms the residual and the red
-// values of plane z, the black values of plane z-1 and the restricted
-// residual of plane z-2 in the same step, so every input plane is read from
-// HBM once.  A stage needs its neighbours' results, so each stage runs on a
-// region one cell wider than the next: the red values cover the tile with a
-// 2-cell halo, the black values a 1-cell halo, the residual the tile itself.
-// Halo cells are recomputed by both neighbouring tiles from the same inputs
-// in the same order, so the values agree bit for bit.
+// Three half-steps instead of two (red and black down, black and red up) cut
+// the CG iterations by a third to a half (column 160x120x96, periodic y: 12 ->
+// 8 at a quarter of the stopping residual).
+// Both march a 64 x 32 (x, y) tile along z (64 x 16 with FP32 records).  The
+// stages of one pass run as a pipeline over planes: in one step the
+// pre-smoothing pass forms the residual and the first red values of plane z,
+// the black values of plane z-1, the second red values of plane z-3 and the
+// restricted residual of plane z-4, so every input plane is read from HBM
+// once.  A stage needs its neighbours' results, so each stage runs on a region
+// one cell wider than the next: the first red values cover the tile with a
+// 3-cell halo, the residual the tile itself.  Halo cells are recomputed by both
+// neighbouring tiles from the same inputs in the same order, so the values
+// agree bit for bit.  The first and third stages do not touch each other's
+// planes, nor do the second and the last: two barriers per plane.
 //
 // Work is split in quads, four consecutive cells x0-4+4q .. x0-1+4q of a
 // row.  x0-4 is even, so in a quad the cells of one colour are the two cells
@@ -29,7 +35,7 @@
 // zero-filling 16-byte cp.async (the records in HBM use the same split along
 // whole grid rows, so a staged half row is one contiguous run); the red
 // stage's vector inputs go to registers, loaded once the stage has consumed
-// the previous plane's.  Three barriers per plane.
+// the previous plane's.
 //
 // The smoother reads per-cell records (beta_x, beta_y, beta_z of the low
 // faces, diagonal) prepared once per coefficient set, the diagonal rounded
@@ -49,24 +55,24 @@ namespace {
 using namespace staged;
 using namespace fused;
 
-// Tile rows: 16 with 8-byte (FP16/BF16) records, 8 with 16-byte (FP32)
-// records, so that three blocks fit the shared memory of an SM.
+// Tile rows: 32 with 8-byte (FP16/BF16) records, 16 with 16-byte (FP32)
+// records; the plane rings fill the shared memory of an SM with one block.
 template <int FTY_>
 struct Geo {
-    static constexpr int FTY = FTY_;               // one thread row per tile row
-    static constexpr int FT = QX * FTY;            // threads per block
-    static constexpr int RH = FTY + 4;             // vector rows:  y0-2 .. y0+FTY+1
-    static constexpr int CH = FTY + 5;             // record rows:  y0-2 .. y0+FTY+2
-    static constexpr int NRED = RH * NQ;           // red-stage quads (rows y0-2 .. y0+FTY+1)
-    static constexpr int NBLK = (FTY + 2) * NQ;    // black-stage quads (rows y0-1 .. y0+FTY)
-    static_assert(NRED <= 2 * FT && NBLK <= 2 * FT, "two tasks per thread");
+    static constexpr int FTY = FTY_;
+    static constexpr int FT = QX * FTY;            // threads per block, one thread row per tile row
+    static constexpr int RH = FTY + 6;             // staged rows: y0-3 .. y0+FTY+2
+    static constexpr int N3 = RH * NQ;             // quads of the 3-halo, 2-halo and 1-halo rows
+    static constexpr int N2 = (RH - 2) * NQ;
+    static constexpr int N1 = (RH - 4) * NQ;
+    static_assert(N3 <= 2 * FT, "two tasks per thread");
 };
 template <int CK>
-using GeoOf = Geo<CK == 0 ? 8 : 16>;
+using GeoOf = Geo<CK == 0 ? 16 : 32>;
 
 // A thread's share of one plane's record copies, resolved once per block:
-// NCT 16-byte copies of the record rows (21 rows x 2 half rows x 36
-// 8-byte records, or 13 rows x 2 x 36 16-byte records).  A copy of two 8-byte
+// NCT 16-byte copies of the record rows (38 rows x 2 half rows x 36
+// 8-byte records, or 22 rows x 2 x 36 16-byte records).  A copy of two 8-byte
 // records covers cells x and x+2 of a quad, so both exist or neither does
 // (nx is a multiple of 4).
 template <int CK>
@@ -76,7 +82,7 @@ struct RecordFetch {
     static constexpr int FT = G::FT;
     static constexpr int RPC = (CK == 0) ? 1 : 2;  // records per 16-byte copy
     static constexpr int PER = HW / RPC;           // copies per half row
-    static constexpr int NCTOT = G::CH * 2 * PER;
+    static constexpr int NCTOT = G::RH * 2 * PER;
     static constexpr int NCT = (NCTOT + FT - 1) / FT;
     int coff[NCT];
     short cdst[NCT];
@@ -100,8 +106,8 @@ struct RecordFetch {
                 const int row = k / (2 * PER), rem = k - row * 2 * PER;
                 const int h = rem / PER, ci = rem - h * PER;
                 bool okx, oky;
-                const int sx = axis_src(x0 - XO + 2 * RPC * ci, g.nx, px, &okx);  // even cell of the copy
-                const int sy = axis_src(y0 - 2 + row, g.ny, py, &oky);
+                const int sx = axis_wrap(x0 - XO + 2 * RPC * ci, g.nx, px, &okx);  // even cell of the copy
+                const int sy = axis_wrap(y0 - 3 + row, g.ny, py, &oky);
                 cok[j] = okx && oky;
                 coff[j] = cok[j] ? g.nx * sy + h * (g.nx >> 1) + (sx >> 1) : 0;
                 cdst[j] = (short)(row * RW + h * HW + RPC * ci);
@@ -109,7 +115,7 @@ struct RecordFetch {
         }
     }
     __device__ __forceinline__ long long plane(int zz, bool* okz) const {
-        const int sz = axis_src(zz, nz, pz, okz);
+        const int sz = axis_wrap(zz, nz, pz, okz);
         return (long long)sz * sxy;
     }
     __device__ __forceinline__ void recs(CT* dst, const CT* src, long long pl, bool okz) const {
@@ -122,73 +128,75 @@ struct RecordFetch {
     }
 };
 
-// A thread's quad tasks of the red / prolongation (2-halo rows, quads 0..17)
-// and black (1-halo rows) stages, resolved once per block: the split-plane
-// offset of the quad's even half (the odd half is HW further), the row's y,
-// the quad's in-plane offset in the grid (wrapped on periodic axes) and
-// whether it exists, and for quads on the tile the unwrapped in-plane offset
-// (-1 otherwise).  Cells outside the regions (quads 0 and 17 reach two cells
-// beyond the 2-halo) are computed like the others and never read.
+// A thread's quad tasks of the first stage (3-halo rows, quads 0..17),
+// resolved once per block: the split-plane offset of the quad's even half (the
+// odd half is HW further), the row's y, the quad's in-plane offset in the grid
+// (wrapped on periodic axes) and whether it exists, and for quads on the tile
+// the unwrapped in-plane offset (-1 otherwise).  The tasks of the second and
+// third half-steps are the same with one and two rows fewer at each end: task
+// k's quad lies one and two rows further (n2, n1: how many of the thread's
+// tasks there are).  Cells outside the regions (quads 0 and 17 reach one cell
+// beyond the 3-halo) are computed like the others and never read.
 template <class G>
 struct QuadTasks {
-    static constexpr int FT = G::FT, FTY = G::FTY, NRED = G::NRED, NBLK = G::NBLK;
+    static constexpr int FT = G::FT, FTY = G::FTY;
     int roff[2], ry[2], rown[2], goff[2];
     bool gok[2];
-    int boff[2], by[2];
+    int n3, n2, n1;
     __device__ __forceinline__ QuadTasks(const Grid3& g, int x0, int y0, int t) {
         const bool px = g.periodic & 1, py = g.periodic & 2;
+        n3 = (t < G::N3) + (t + FT < G::N3);
+        n2 = (t < G::N2) + (t + FT < G::N2);
+        n1 = (t < G::N1) + (t + FT < G::N1);
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int k = t + u * FT;
-            roff[u] = -1;
-            ry[u] = 0;
+            const int row = k / NQ, q = k - row * NQ;
+            roff[u] = row * RW + 2 * q;
+            const int gx = x0 - XO + 4 * q, gy = y0 - 3 + row;
+            ry[u] = gy;
             rown[u] = -1;
-            goff[u] = 0;
-            gok[u] = false;
-            if (k < NRED) {
-                const int row = k / NQ, q = k - row * NQ;
-                roff[u] = row * RW + 2 * q;
-                const int gx = x0 - XO + 4 * q, gy = y0 - 2 + row;
-                ry[u] = gy;
-                if (row >= 2 && row < FTY + 2 && q >= 1 && q <= QX && gx < g.nx && gy < g.ny) rown[u] = gx + g.nx * gy;
-                bool okx, oky;
-                const int sx = axis_src(gx, g.nx, px, &okx);
-                const int sy = axis_src(gy, g.ny, py, &oky);
-                gok[u] = okx && oky;
-                goff[u] = gok[u] ? sx + g.nx * sy : 0;
-            }
-            boff[u] = -1;
-            by[u] = 0;
-            if (k < NBLK) {
-                const int rb = k / NQ, q = k - rb * NQ, row = rb + 1;
-                boff[u] = row * RW + 2 * q;
-                by[u] = y0 - 2 + row;
-            }
+            if (row >= 3 && row < FTY + 3 && q >= 1 && q <= QX && gx < g.nx && gy < g.ny) rown[u] = gx + g.nx * gy;
+            bool okx, oky;
+            const int sx = axis_wrap(gx, g.nx, px, &okx);
+            const int sy = axis_wrap(gy, g.ny, py, &oky);
+            gok[u] = u < n3 && okx && oky;
+            goff[u] = gok[u] ? sx + g.nx * sy : 0;
         }
     }
 };
-// Plane rings in shared memory.  A step handles planes zA (red /
-// prolongation stage), zA-1 (black stage) and zA-2 (tile stage) and stages
-// the records of plane zA+1 for the next step; rings of 4 planes, so the z
-// loop is unrolled four times and every slot is a compile-time offset.  In
-// the correction ring the black cells of the newest plane hold their
-// right-hand side sigma r until the black stage replaces it by their value.
-template <int CK>
-struct PreRing {
+// Plane rings in shared memory, six planes deep; gb: the black cells' right-
+// hand side sigma r, for the stage after the one that overwrites or does not
+// reach it.
+template <int CK, int GP>
+struct PlaneRing {
     using CT = typename CoefStore<CK>::T;
     using G = GeoOf<CK>;
-    CT c[4][G::CH][RW];              // records, planes zA-2 .. zA+1
-    float er[4][G::RH][RW];          // correction, planes zA-3 .. zA
-    float2 ypart[G::FTY][QX];
+    CT c[6][G::RH][RW];              // records, planes zA-4 .. zA+1
+    float e[6][G::RH][RW];           // correction, planes zA-5 .. zA
+    float gb[GP][G::RH][HW];         // planes zA-GP+1 .. zA
 };
 template <int CK>
-struct PostRing {
-    using CT = typename CoefStore<CK>::T;
-    using G = GeoOf<CK>;
-    CT c[4][G::CH][RW];              // records, planes zA-2 .. zA+1
-    float ep[4][G::RH][RW];          // prolonged / smoothed correction, planes zA-3 .. zA
+struct PreRing : PlaneRing<CK, 5> {
+    float2 ypart[GeoOf<CK>::FTY][QX];
 };
-constexpr int FUSED_MIN_BLOCKS = 3;
+template <int CK>
+using PostRing = PlaneRing<CK, 4>;
+// Ring slots (offsets) of planes zA, zA-1, ..
+template <int N>
+struct RingSlots {
+    int s[N];
+    __device__ __forceinline__ RingSlots(int stride) {
+#pragma unroll
+        for (int k = 0; k < N; k++) s[k] = ((N - k) % N) * stride;
+    }
+    __device__ __forceinline__ void advance() {
+        const int last = s[N - 1];
+#pragma unroll
+        for (int k = N - 1; k > 0; k--) s[k] = s[k - 1];
+        s[0] = last;
+    }
+};
 }  // namespace
 
 // ------------------------------------------------------ pre-smoothing pass
@@ -196,13 +204,12 @@ constexpr int FUSED_MIN_BLOCKS = 3;
 // residual rc.  UPDATE (finest level inside CG): the residual is first
 // updated, r_out = rin - alpha q, written for the tile's cells, and ||r_out||^2
 // decides convergence.  FINE: the right-hand side is sigma * r.
-// After the two half-steps the residual of a black cell is zero (its update
-// solves its own equation) and that of a red cell is sum beta * e over its
-// black neighbours (its red value solved the equation with them at zero), so
-// the restriction sums those neighbour terms over the red cells.
+// After the three half-steps the residual of a red cell is zero (its last
+// update solved its own equation), so the restriction sums the black cells'.
+// e receives the black half of the correction, rows of nx/2 values.
 // rin and q must not alias r_out (other tiles read them as halo).
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-__global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
+__global__ void __launch_bounds__(GeoOf<CK>::FT)
     k_presmooth_restrict(Grid3 g, Grid3 gc, const void* __restrict__ sm_v, const VT* __restrict__ rin,
                          const float* __restrict__ q, float* __restrict__ r_out, VT* __restrict__ e,
                          VTc* __restrict__ rc, Scalars* sc, double* partials, int nblocks) {
@@ -230,17 +237,24 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
     int rc_z = -1;  // coarse plane whose restriction awaits the row pair sum
     const int ox = x0 + 4 * tx, oy = y0 + ty;  // the thread's own quad
     const bool own_inside = ox < g.nx && oy < g.ny;
-    const int oo = (ty + 2) * RW + 2 * (tx + 1);  // split offset of its even half
+    const int oo = (ty + 3) * RW + 2 * (tx + 1);  // split offset of its even half
+    const int ob = (ty + 3) * HW + 2 * (tx + 1);  // its offset in the black planes
     const long long og = ox + (long long)g.nx * oy;
+    CT* const cb = &S.c[0][0][0];
+    float* const eb = &S.e[0][0][0];
+    float* const gb = &S.gb[0][0][0];
+    constexpr int SLOT = G::RH * RW;
+    RingSlots<6> R(SLOT);
+    RingSlots<5> RG(G::RH * HW);
     R4 rv[2];
     float4 qv[2];
-    auto stage = [&](int zz, int c4) {
+    auto stage = [&](int zz, int off) {
         bool okz;
         const long long pl = F.plane(zz, &okz);
-        F.recs(&S.c[c4][0][0], sm, pl, okz);
+        F.recs(cb + off, sm, pl, okz);
         cp_commit();
     };
-    auto load = [&](int zz) {  // the red tasks' residual (and q) of plane zz
+    auto load = [&](int zz) {  // the first stage's residual (and q) of plane zz
         bool okz;
         const long long pl = F.plane(zz, &okz);
 #pragma unroll
@@ -258,22 +272,25 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
         }
         rc_z = -1;
     };
-    auto step = [&](auto ph, int zA) {
-        constexpr int P = decltype(ph)::value;
+    const int zs = z0 - 3, zend = z1 + 3;
+    stage(zs, 0);
+    load(zs);
+    for (int zA = zs; zA <= zend; zA++) {
         cp_wait<0>();
         __syncthreads();
-        stage(zA + 1, (P + 1) & 3);
+        if (zA < z1 + 2) stage(zA + 1, R.s[5]);
         flush_rc();
-        // ---- red stage: plane zA over the 2-halo rows
-        {
-            const CT* C = &S.c[P][0][0];
-            float* ER = &S.er[P][0][0];
+        // ---- first red half-step: plane zA over the 3-halo rows
+        if (zA <= z1 + 2) {
+            const CT* C = cb + R.s[0];
+            float* E = eb + R.s[0];
+            float* GB = gb + RG.s[0];
             const bool zin = zA >= z0 && zA < z1;
             float* rplane = UPDATE ? r_out + sxy * zA : nullptr;
 #pragma unroll
             for (int u = 0; u < 2; u++) {
+                if (u >= T.n3) break;
                 const int o = T.roff[u];
-                if (o < 0) break;
                 float4 rn = cvt4r<VT>(rv[u]);
                 if (UPDATE)
                     rn = make_float4(fmaf(-alpha, qv[u].x, rn.x), fmaf(-alpha, qv[u].y, rn.y),
@@ -283,107 +300,86 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
                 rec2<CK>(C + o + p * HW, &d0, &d1);
                 const float2 rr = p ? make_float2(rn.y, rn.w) : make_float2(rn.x, rn.z);  // red cells
                 const float2 rb = p ? make_float2(rn.x, rn.z) : make_float2(rn.y, rn.w);  // black cells
-                const float2 ev = divide2(make_float2(sigma * rr.x, sigma * rr.y), make_float2(d0.w, d1.w));
-                *reinterpret_cast<float2*>(ER + o + p * HW) = ev;
-                *reinterpret_cast<float2*>(ER + o + (1 - p) * HW) = make_float2(sigma * rb.x, sigma * rb.y);
+                *reinterpret_cast<float2*>(E + o + p * HW) =
+                    divide2(make_float2(sigma * rr.x, sigma * rr.y), make_float2(d0.w, d1.w));
+                *reinterpret_cast<float2*>(GB + half_off(o)) = make_float2(sigma * rb.x, sigma * rb.y);
                 if (UPDATE && zin && T.rown[u] >= 0) {
                     *reinterpret_cast<float4*>(rplane + T.rown[u]) = rn;
                     rr_thread = fmaf(rn.x, rn.x, fmaf(rn.y, rn.y, fmaf(rn.z, rn.z, fmaf(rn.w, rn.w, rr_thread))));
                 }
             }
+            if (zA < z1 + 2) load(zA + 1);
         }
-        load(zA + 1);
-        __syncthreads();
-        // ---- black stage: plane zA-1 over the 1-halo rows, in place
-        const int zB = zA - 1;
-        if (zB >= z0 - 1) {
-            const CT* C = &S.c[(P + 3) & 3][0][0];
-            const CT* CN = &S.c[P][0][0];
-            float* E = &S.er[(P + 3) & 3][0][0];
-            const float* EM = &S.er[(P + 2) & 3][0][0];
-            const float* EP = &S.er[P][0][0];
+        // ---- second red half-step: plane zA-3 over the 1-halo rows
+        const int z3 = zA - 3;
+        if (z3 >= z0 - 1) {
+            float* E = eb + R.s[3];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                if (T.boff[u] < 0) break;
-                const int h = 1 - red_half(T.by[u], zB);
-                const int o = T.boff[u] + h * HW;
+                if (u >= T.n1) break;
+                const int h = red_half(T.ry[u] + 2, z3);
+                const int o = T.roff[u] + 2 * RW + h * HW;
                 float2 d;
-                const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, o, h, *reinterpret_cast<const float2*>(E + o), &d);
-                *reinterpret_cast<float2*>(E + o) = divide2(s, d);
+                const float2 s = gs_sum2<CK>(cb + R.s[3], cb + R.s[2], E, eb + R.s[4], eb + R.s[2], o, h,
+                                             make_float2(0.f, 0.f), &d);
+                const float2 dv = divide2(s, d), ev = *reinterpret_cast<const float2*>(E + o);
+                *reinterpret_cast<float2*>(E + o) = make_float2(ev.x + dv.x, ev.y + dv.y);
             }
         }
         __syncthreads();
-        // ---- correction out and restriction: plane zA-2 over the tile
-        const int zC = zA - 2;
-        if (zC >= z0 && zC < z1) {
-            const CT* C = &S.c[(P + 2) & 3][0][0];
-            const CT* CN = &S.c[(P + 3) & 3][0][0];
-            const float* E = &S.er[(P + 2) & 3][0][0];
-            const float* EM = &S.er[(P + 1) & 3][0][0];
-            const float* EP = &S.er[(P + 3) & 3][0][0];
-            const int p = red_half(oy, zC);  // red half of the own quad
-            float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, oo + p * HW, p, make_float2(0.f, 0.f), &d);
-            part.x += s.x;
-            part.y += s.y;
-            if (own_inside) {
-                const float2 ev = *reinterpret_cast<const float2*>(E + oo);
-                const float2 od = *reinterpret_cast<const float2*>(E + oo + HW);
-                st4<VT>(e + (og + sxy * zC), make_float4(ev.x, od.x, ev.y, od.y));
+        // ---- black half-step: plane zA-1 over the 2-halo rows
+        const int zB = zA - 1;
+        if (zB >= z0 - 2 && zB <= z1 + 1) {
+            float* E = eb + R.s[1];
+            const float* GB = gb + RG.s[1];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (u >= T.n2) break;
+                const int h = 1 - red_half(T.ry[u] + 1, zB);
+                const int o = T.roff[u] + RW + h * HW;
+                float2 d;
+                const float2 s = gs_sum2<CK>(cb + R.s[1], cb + R.s[0], E, eb + R.s[2], eb + R.s[0], o, h,
+                                             *reinterpret_cast<const float2*>(GB + half_off(T.roff[u]) + HW), &d);
+                const float2 v = divide2(s, d);
+                *reinterpret_cast<float2*>(E + o) = make_float2(SOR_BLACK * v.x, SOR_BLACK * v.y);
             }
-            if (((zC - z0) & 1) || zC + 1 == z1) {
+        }
+        // ---- correction out and restriction: plane zA-4 over the tile
+        const int zD = zA - 4;
+        if (zD >= z0) {
+            const float* E = eb + R.s[4];
+            const int h = 1 - red_half(oy, zD);  // black half of the own quad
+            const float2 gv = *reinterpret_cast<const float2*>(gb + RG.s[4] + ob);
+            const float2 bv = *reinterpret_cast<const float2*>(E + oo + h * HW);
+            float2 d;
+            const float2 s = gs_sum2<CK>(cb + R.s[4], cb + R.s[3], E, eb + R.s[5], eb + R.s[3], oo + h * HW, h, gv, &d);
+            part.x += fmaf(-d.x, bv.x, s.x);
+            part.y += fmaf(-d.y, bv.y, s.y);
+            if (own_inside) st2<VT>(e + ((og + sxy * zD) >> 1), bv);
+            if (((zD - z0) & 1) || zD + 1 == z1) {
                 // the row pair sum is formed after the next barrier
                 S.ypart[ty][tx] = part;
-                rc_z = zC >> 1;
+                rc_z = zD >> 1;
                 part = make_float2(0.f, 0.f);
             }
         }
-    };
-    const int zs = z0 - 2, zend = z1 + 1;  // red stage over zs .. zend
-    stage(zs, 0);
-    load(zs);
-    for (int zA = zs;;) {
-        step(Phase<0>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<1>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<2>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<3>{}, zA);
-        if (++zA > zend) break;
+        R.advance();
+        RG.advance();
     }
     cp_wait<0>();
     __syncthreads();
     flush_rc();
-    if (UPDATE) {
-        double v1[1] = {(double)rr_thread};
-        block_sum<1>(v1, sh);
-        if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[8])) {
-            double tot[1];
-            finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[8]);
-            if (t == 0) {
-                const double rr = tot[0];
-                sc->rr = rr;
-                sc->iterations += 1;
-                sc->total_iterations += 1;
-                if (!isfinite(rr)) {
-                    sc->nonfinite = 1;
-                    sc->converged = 1;
-                } else if (rr <= sc->rr_target || sc->total_iterations >= sc->max_total) {
-                    sc->converged = 1;
-                }
-            }
-        }
-    }
+    if (UPDATE) finish_residual_norm(rr_thread, sc, partials, nblocks, sh);
 }
 
 // ----------------------------------------------------- post-smoothing pass
-// e (pre-smoothed, VT) + w * P ec -> black, red half-steps -> out (VT).  DOT
-// (finest level): r . out / sigma gives rz and beta; the next V-cycle's sigma
-// is then taken from ||r||^2.  The black half-step does not read a black
-// cell's own prolonged value, so the prolongation stage leaves sigma r there.
+// e (pre-smoothed black half, VT) + w * P ec -> red, black, red half-steps ->
+// out (VT).  DOT (finest level): r . out / sigma gives rz and beta; the next
+// V-cycle's sigma is then taken from ||r||^2.  The first half-step does not
+// read a red cell's own prolonged value, so the prolongation stage leaves
+// sigma r there.
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
-__global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
+__global__ void __launch_bounds__(GeoOf<CK>::FT)
     k_prolong_postsmooth(Grid3 g, Grid3 gc, const void* __restrict__ sm_v, const VT* __restrict__ e,
                          const VTc* __restrict__ ec, const VT* __restrict__ r, VT* __restrict__ out,
                          const VT* __restrict__ accum, float w, Scalars* sc, double* partials, int nblocks,
@@ -393,6 +389,7 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
     using G = GeoOf<CK>;
     constexpr int FTY = G::FTY, FT = G::FT;
     using R4 = typename Raw4<VT>::T;
+    using V2 = typename Raw2<VT>::T;
     using C2 = typename Raw2<VTc>::T;
     const CT* sm = reinterpret_cast<const CT*>(sm_v);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -406,121 +403,139 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
     const RecordFetch<CK> F(g, x0, y0, t);
     const QuadTasks<G> T(g, x0, y0, t);
     const long long sxy = (long long)g.nx * g.ny;
-    // coarse parents of the red-stage quads: in-plane offsets of the pair
+    // coarse parents of the first stage's quads: in-plane offsets of the pair
     int pofs[2];
     {
         const bool px = g.periodic & 1, py = g.periodic & 2;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int k = t + u * FT;
-            pofs[u] = 0;
-            if (k < G::NRED) {
-                const int row = k / NQ, qq = k - row * NQ;
-                bool okx, oky;
-                const int sx = axis_src(x0 - XO + 4 * qq, g.nx, px, &okx);
-                const int sy = axis_src(y0 - 2 + row, g.ny, py, &oky);
-                pofs[u] = (okx && oky) ? (sx >> 1) + gc.nx * (sy >> 1) : 0;
-            }
+            const int row = k / NQ, qq = k - row * NQ;
+            bool okx, oky;
+            const int sx = axis_wrap(x0 - XO + 4 * qq, g.nx, px, &okx);
+            const int sy = axis_wrap(y0 - 3 + row, g.ny, py, &oky);
+            pofs[u] = T.gok[u] ? (sx >> 1) + gc.nx * (sy >> 1) : 0;
         }
     }
     const long long csxy = (long long)gc.nx * gc.ny;
     Acc acc;
     const int ox = x0 + 4 * tx, oy = y0 + ty;
     const bool own_inside = ox < g.nx && oy < g.ny;
-    const int oo = (ty + 2) * RW + 2 * (tx + 1);
+    const int oo = (ty + 3) * RW + 2 * (tx + 1);
     const long long og = ox + (long long)g.nx * oy;
-    // registers of the red-stage quads of the next plane: the pre-smoothed
-    // correction, the right-hand side (for the black cells) and the coarse
+    CT* const cb = &S.c[0][0][0];
+    float* const eb = &S.e[0][0][0];
+    float* const gb = &S.gb[0][0][0];
+    constexpr int SLOT = G::RH * RW;
+    RingSlots<6> R(SLOT);
+    RingSlots<4> RG(G::RH * HW);
+    // registers of the first stage's quads of the next plane: the black half
+    // of the pre-smoothed correction, the right-hand side and the coarse
     // parents; and the own quad's right-hand side of the tile plane
-    R4 eov[2], rqv[2];
+    V2 eov[2];
+    R4 rqv[2];
     C2 pcv[2];
-    R4 rov, ron;
-    auto stage = [&](int zz, int c4) {
+    R4 rov;
+    auto stage = [&](int zz, int off) {
         bool okz;
         const long long pl = F.plane(zz, &okz);
-        F.recs(&S.c[c4][0][0], sm, pl, okz);
+        F.recs(cb + off, sm, pl, okz);
         cp_commit();
     };
     auto load = [&](int zz) {
         bool okz;
-        const int sz = axis_src(zz, g.nz, (g.periodic & 4) != 0, &okz);
+        const int sz = axis_wrap(zz, g.nz, (g.periodic & 4) != 0, &okz);
         const long long pl = (long long)sz * sxy, cpl = (long long)(sz >> 1) * csxy;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const bool ok = T.gok[u] && okz;
-            eov[u] = ldg_quad<VT>(e + pl + T.goff[u], ok);
+            eov[u] = ldg_pair<VT>(e + ((pl + T.goff[u]) >> 1), ok);
             rqv[u] = ldg_quad<VT>(r + pl + T.goff[u], ok);
             pcv[u] = ldg_pair<VTc>(ec + cpl + pofs[u], ok);
         }
-        const int zt = zz - 2;  // the tile plane of the step that uses this plane's red stage
-        ron = ldg_quad<VT>(r + og + sxy * zt, own_inside && zt >= z0 && zt < z1);
     };
-    auto step = [&](auto ph, int zA) {
-        constexpr int P = decltype(ph)::value;
+    const int zs = z0 - 3, zend = z1 + 3;
+    stage(zs, 0);
+    load(zs);
+    for (int zA = zs; zA <= zend; zA++) {
         cp_wait<0>();
         __syncthreads();
-        stage(zA + 1, (P + 1) & 3);
-        rov = ron;
-        // ---- prolongation: plane zA over the 2-halo rows
-        {
-            float* EP = &S.ep[P][0][0];
+        if (zA < z1 + 2) stage(zA + 1, R.s[5]);
+        const int zD = zA - 4;
+        rov = ldg_quad<VT>(r + og + sxy * zD, own_inside && zD >= z0);
+        // ---- prolongation: plane zA over the 3-halo rows
+        if (zA <= z1 + 2) {
+            float* E = eb + R.s[0];
+            float* GB = gb + RG.s[0];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
+                if (u >= T.n3) break;
                 const int o = T.roff[u];
-                if (o < 0) break;
-                const float4 ev = cvt4r<VT>(eov[u]);
+                const float2 ev = cvt2(eov[u]);
                 const float4 rq = cvt4r<VT>(rqv[u]);
                 const float2 cv = cvt2(pcv[u]);
                 const int p = red_half(T.ry[u], zA);
-                const float2 er = p ? make_float2(ev.y, ev.w) : make_float2(ev.x, ev.z);
+                const float2 rr = p ? make_float2(rq.y, rq.w) : make_float2(rq.x, rq.z);
                 const float2 rb = p ? make_float2(rq.x, rq.z) : make_float2(rq.y, rq.w);
-                *reinterpret_cast<float2*>(EP + o + p * HW) = make_float2(fmaf(w, cv.x, er.x), fmaf(w, cv.y, er.y));
-                *reinterpret_cast<float2*>(EP + o + (1 - p) * HW) = make_float2(sigma * rb.x, sigma * rb.y);
+                *reinterpret_cast<float2*>(E + o + p * HW) = make_float2(sigma * rr.x, sigma * rr.y);
+                *reinterpret_cast<float2*>(E + o + (1 - p) * HW) = make_float2(fmaf(w, cv.x, ev.x), fmaf(w, cv.y, ev.y));
+                *reinterpret_cast<float2*>(GB + half_off(o)) = make_float2(sigma * rb.x, sigma * rb.y);
             }
+            if (zA < z1 + 2) load(zA + 1);
         }
-        load(zA + 1);
-        __syncthreads();
-        // ---- black half-step: plane zA-1 over the 1-halo rows, in place
-        const int zB = zA - 1;
-        if (zB >= z0 - 1) {
-            const CT* C = &S.c[(P + 3) & 3][0][0];
-            const CT* CN = &S.c[P][0][0];
-            float* E = &S.ep[(P + 3) & 3][0][0];
-            const float* EM = &S.ep[(P + 2) & 3][0][0];
-            const float* EP = &S.ep[P][0][0];
+        // ---- black half-step: plane zA-3 over the 1-halo rows
+        const int z3 = zA - 3;
+        if (z3 >= z0 - 1) {
+            float* E = eb + R.s[3];
+            const float* GB = gb + RG.s[3];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                if (T.boff[u] < 0) break;
-                const int h = 1 - red_half(T.by[u], zB);
-                const int o = T.boff[u] + h * HW;
+                if (u >= T.n1) break;
+                const int h = 1 - red_half(T.ry[u] + 2, z3);
+                const int o = T.roff[u] + 2 * RW + h * HW;
                 float2 d;
-                const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, o, h, *reinterpret_cast<const float2*>(E + o), &d);
+                const float2 s = gs_sum2<CK>(cb + R.s[3], cb + R.s[2], E, eb + R.s[4], eb + R.s[2], o, h,
+                                             *reinterpret_cast<const float2*>(GB + half_off(T.roff[u]) + 2 * HW), &d);
+                const float2 v = divide2(s, d), pv = *reinterpret_cast<const float2*>(E + o);
+                *reinterpret_cast<float2*>(E + o) =
+                    make_float2(d.x > 0.f ? fmaf(SOR_BLACK, v.x - pv.x, pv.x) : 0.f,
+                                d.y > 0.f ? fmaf(SOR_BLACK, v.y - pv.y, pv.y) : 0.f);
+            }
+        }
+        __syncthreads();
+        // ---- first red half-step: plane zA-1 over the 2-halo rows, in place
+        const int zB = zA - 1;
+        if (zB >= z0 - 2 && zB <= z1 + 1) {
+            float* E = eb + R.s[1];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (u >= T.n2) break;
+                const int h = red_half(T.ry[u] + 1, zB);
+                const int o = T.roff[u] + RW + h * HW;
+                float2 d;
+                const float2 s = gs_sum2<CK>(cb + R.s[1], cb + R.s[0], E, eb + R.s[2], eb + R.s[0], o, h,
+                                             *reinterpret_cast<const float2*>(E + o), &d);
                 *reinterpret_cast<float2*>(E + o) = divide2(s, d);
             }
         }
-        __syncthreads();
-        // ---- red half-step: plane zA-2 over the tile, out = z
-        const int zC = zA - 2;
-        if (zC >= z0 && zC < z1) {
-            const CT* C = &S.c[(P + 2) & 3][0][0];
-            const CT* CN = &S.c[(P + 3) & 3][0][0];
-            const float* E = &S.ep[(P + 2) & 3][0][0];
-            const float* EM = &S.ep[(P + 1) & 3][0][0];
-            const float* EP = &S.ep[(P + 3) & 3][0][0];
-            const int p = red_half(oy, zC);
+        // ---- second red half-step: plane zA-4 over the tile, out = z
+        if (zD >= z0) {
+            const float* E = eb + R.s[4];
+            const int p = red_half(oy, zD);
             const float4 rv = cvt4r<VT>(rov);
             const float2 rr = p ? make_float2(rv.y, rv.w) : make_float2(rv.x, rv.z);
             float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, oo + p * HW, p, make_float2(sigma * rr.x, sigma * rr.y), &d);
+            const float2 s = gs_sum2<CK>(cb + R.s[4], cb + R.s[3], E, eb + R.s[5], eb + R.s[3], oo + p * HW, p,
+                                         make_float2(sigma * rr.x, sigma * rr.y), &d);
             const float2 zr = divide2(s, d);
             const float2 zb = *reinterpret_cast<const float2*>(E + oo + (1 - p) * HW);
             float4 zv = p ? make_float4(zb.x, zr.x, zb.y, zr.y) : make_float4(zr.x, zb.x, zr.y, zb.y);
             if (own_inside) {
                 if (accum) {  // out = accum + z (second W-cycle visit)
-                    const float4 a = cvt4r<VT>(*reinterpret_cast<const R4*>(accum + og + sxy * zC));
+                    const float4 a = cvt4r<VT>(*reinterpret_cast<const R4*>(accum + og + sxy * zD));
                     zv = make_float4(a.x + zv.x, a.y + zv.y, a.z + zv.z, a.w + zv.w);
                 }
-                st4<VT>(out + og + sxy * zC, zv);
+                st4<VT>(out + og + sxy * zD, zv);
                 if (DOT) {
                     acc.add_prod(rv.x, zv.x * is);
                     acc.add_prod(rv.y, zv.y * is);
@@ -529,51 +544,11 @@ __global__ void __launch_bounds__(GeoOf<CK>::FT, FUSED_MIN_BLOCKS)
                 }
             }
         }
-    };
-    const int zs = z0 - 2, zend = z1 + 1;
-    stage(zs, 0);
-    load(zs);
-    for (int zA = zs;;) {
-        step(Phase<0>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<1>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<2>{}, zA);
-        if (++zA > zend) break;
-        step(Phase<3>{}, zA);
-        if (++zA > zend) break;
+        R.advance();
+        RG.advance();
     }
     cp_wait<0>();
-    if (DOT) {
-        double v1[1] = {acc.total()};
-        block_sum<1>(v1, sh);
-        if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[9])) {
-            double tot[1];
-            finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[9]);
-            if (t == 0) {
-                const double rz = tot[0];
-                if (!isfinite(rz)) {
-                    sc->nonfinite = 1;
-                    sc->converged = 1;
-                } else if (!(rz > 0.0)) {
-                    sc->breakdown = 1;
-                    sc->converged = 1;
-                } else if (sc->first) {
-                    sc->rz = rz;
-                    sc->beta = 0.0;
-                    sc->beta_f = 0.0f;
-                } else {
-                    sc->beta = rz / sc->rz;
-                    sc->beta_f = (float)sc->beta;
-                    sc->rz = rz;
-                }
-                // z is in units of this V-cycle's sigma; the next V-cycle
-                // scales by the RMS of the residual it will be given.
-                sc->inv_sigma_z = sc->inv_sigma;
-                set_sigma_from(sc, sc->rr, n_active);
-            }
-        }
-    }
+    if (DOT) finish_rz(acc.total(), sc, partials, nblocks, n_active, sh);
 }
 
 // --------------------------------------------------- smoother records
@@ -629,7 +604,7 @@ int f_occ[12] = {};
 enum { O_PRE_F32 = 0, O_PRE_LO, O_PRE_LO_UPD, O_PRE_F32_UPD, O_PRE_COARSE, O_POST_F32, O_POST_LO, O_POST_COARSE };
 
 // Even z runs chosen so the grid fills whole waves of resident blocks; each
-// run also computes two planes below and above it.  On levels too small to
+// run also computes three planes below and above it and drains one step.  On levels too small to
 // fill one wave the score favours the shortest runs (fewest steps per block).
 Launch fused_launch(const Grid3& g0, int occ_kind, int fty) {
     Launch P;
@@ -648,7 +623,7 @@ Launch fused_launch(const Grid3& g0, int occ_kind, int fty) {
         const long long blocks = (long long)tiles * zcr;
         if (blocks > MAX_REDUCE_BLOCKS) break;
         const double waves = (double)blocks / cap;
-        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 4));
+        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 7));
         if (score > best) {
             best = score;
             best_zper = zper;
@@ -672,18 +647,29 @@ bool fused_supported(const Grid3& g) {
 }
 
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-static void pre_impl(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q, float* r_out,
-                     void* e, void* rc, Scalars* sc, double* partials, int occ_kind, cudaStream_t s) {
-    if (tma_pre(CK, FINE, UPDATE, g, gc, sm, rin, q, r_out, e, rc, sc, partials, s)) return;
+static void pre_impl(const MGLevel& lv, const Grid3& gc, const void* rin, const float* q, float* r_out, void* e,
+                     void* rc, Scalars* sc, double* partials, int occ_kind, cudaStream_t s) {
+    const Grid3& g = lv.L.g;
+    const void* sm = lv.sm;
+    if (lv.passes == PASS_TMA) return tma_pre(CK, FINE, UPDATE, g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
+    if (lv.passes == PASS_PAIR) return pair_pre(FINE, UPDATE, g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
+    if (lv.passes == PASS_RUN) return run_pre(CK, FINE, UPDATE, g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
     const Launch P = fused_launch(g, occ_kind, GeoOf<CK>::FTY);
     k_presmooth_restrict<CK, VT, VTc, UPDATE, FINE><<<P.grid, P.block, sizeof(PreRing<CK>), s>>>(
         P.g, gc, sm, (const VT*)rin, q, r_out, (VT*)e, (VTc*)rc, sc, partials, P.nblocks);
 }
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
-static void post_impl(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r,
-                      void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active,
-                      int occ_kind, cudaStream_t s) {
-    if (tma_post(CK, FINE, g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s)) return;
+static void post_impl(const MGLevel& lv, const Grid3& gc, const void* e, const void* ec, const void* r, void* out,
+                      const void* accum, float w, Scalars* sc, double* partials, long long n_active, int occ_kind,
+                      cudaStream_t s) {
+    const Grid3& g = lv.L.g;
+    const void* sm = lv.sm;
+    if (lv.passes == PASS_TMA)
+        return tma_post(CK, FINE, g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
+    if (lv.passes == PASS_PAIR)
+        return pair_post(FINE, g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
+    if (lv.passes == PASS_RUN)
+        return run_post(CK, FINE, g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
     const Launch P = fused_launch(g, occ_kind, GeoOf<CK>::FTY);
     k_prolong_postsmooth<CK, VT, VTc, DOT, FINE><<<P.grid, P.block, sizeof(PostRing<CK>), s>>>(
         P.g, gc, sm, (const VT*)e, (const VTc*)ec, (const VT*)r, (VT*)out, (const VT*)accum, w, sc, partials,
@@ -737,16 +723,18 @@ static const void* fused_solve_level(const MGPlan& P, int l, double* partials, l
     }
     const MGLevel &L = P.lv[l], &C = P.lv[l + 1];
     auto visit = [&](const void* rhs, void* out, const void* accum) {
-        pre_impl<CK, VT, VT, false, false>(L.L.g, C.L.g, L.sm, rhs, nullptr, nullptr, L.e, C.r, P.sc, partials,
+        pre_impl<CK, VT, VT, false, false>(L, C.L.g, rhs, nullptr, nullptr, L.e, C.r, P.sc, partials,
                                            O_PRE_COARSE, s);
         const void* ec = fused_solve_level<CK, VT>(P, l + 1, partials, n_active, s);
-        post_impl<CK, VT, VT, false, false>(L.L.g, C.L.g, L.sm, L.e, ec, rhs, out, accum, P.prolong, P.sc, partials,
+        post_impl<CK, VT, VT, false, false>(L, C.L.g, L.e, ec, rhs, out, accum, P.prolong, P.sc, partials,
                                             n_active, O_POST_COARSE, s);
     };
     visit(L.r, L.eo, nullptr);
     if (P.w_from > 0 && l >= P.w_from && l <= P.w_to) {
-        k_level_residual<CK, VT><<<L.L.grid, L.L.block, 0, s>>>(L.L.g, L.sm, (const VT*)L.r, (const VT*)L.eo,
-                                                               (VT*)L.r2, P.sc);
+        if (L.passes == PASS_TMA) tma_level_residual(CK, L.L, L.sm, L.r, L.eo, L.r2, P.sc, s);
+        else
+            k_level_residual<CK, VT><<<L.L.grid, L.L.block, 0, s>>>(L.L.g, L.sm, (const VT*)L.r, (const VT*)L.eo,
+                                                                   (VT*)L.r2, P.sc);
         visit(L.r2, L.eo2, L.eo);
         return L.eo2;
     }
@@ -757,13 +745,13 @@ template <int CK, class VT>
 static void vcycle_fused_impl(const MGPlan& P, const float* r_in, const float* q, float* r_out, bool update,
                               double* partials, long long n_active, cudaStream_t s) {
     if (update)
-        pre_impl<CK, float, VT, true, true>(P.lv[0].L.g, P.lv[1].L.g, P.lv[0].sm, r_in, q, r_out, P.e0, P.lv[1].r,
+        pre_impl<CK, float, VT, true, true>(P.lv[0], P.lv[1].L.g, r_in, q, r_out, P.e0, P.lv[1].r,
                                             P.sc, partials, CK == 0 ? O_PRE_F32_UPD : O_PRE_LO_UPD, s);
     else
-        pre_impl<CK, float, VT, false, true>(P.lv[0].L.g, P.lv[1].L.g, P.lv[0].sm, r_in, nullptr, nullptr, P.e0,
+        pre_impl<CK, float, VT, false, true>(P.lv[0], P.lv[1].L.g, r_in, nullptr, nullptr, P.e0,
                                              P.lv[1].r, P.sc, partials, CK == 0 ? O_PRE_F32 : O_PRE_LO, s);
     const void* ec1 = fused_solve_level<CK, VT>(P, 1, partials, n_active, s);
-    post_impl<CK, float, VT, true, true>(P.lv[0].L.g, P.lv[1].L.g, P.lv[0].sm, P.e0, ec1, update ? r_out : r_in,
+    post_impl<CK, float, VT, true, true>(P.lv[0], P.lv[1].L.g, P.e0, ec1, update ? r_out : r_in,
                                          P.lv[0].e, nullptr, P.prolong, P.sc, partials, n_active,
                                          CK == 0 ? O_POST_F32 : O_POST_LO, s);
 }
@@ -780,7 +768,8 @@ static void records_impl(const MGPlan& P, cudaStream_t s) {
     for (int l = 0; l < P.fused_levels; l++) {
         const MGLevel& L = P.lv[l];
         const void* coef = CK == 0 ? (const void*)L.coef32 : L.coef_lo;
-        k_smoother_records<CK><<<L.L.grid, L.L.block, 0, s>>>(L.L.g, coef, L.sm);
+        if (L.passes == PASS_TMA) tma_records(CK, L.L, coef, L.sm, s);
+        else k_smoother_records<CK><<<L.L.grid, L.L.block, 0, s>>>(L.L.g, coef, L.sm);
     }
 }
 void mg_smoother_records(const MGPlan& P, cudaStream_t s) {
@@ -801,47 +790,45 @@ void mg_fused_coarse(const MGPlan& P, double* partials, long long n_active, cuda
 // Single passes, for measurement.
 void mg_fused_pre(const MGPlan& P, const float* r_in, const float* q, float* r_out, double* partials,
                   cudaStream_t s) {
-    const Grid3 &g = P.lv[0].L.g, &gc = P.lv[1].L.g;
-    const void* sm = P.lv[0].sm;
+    const MGLevel& lv = P.lv[0];
+    const Grid3& gc = P.lv[1].L.g;
     if (P.precision == 1)
-        pre_impl<1, float, __half, true, true>(g, gc, sm, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials, O_PRE_LO_UPD, s);
+        pre_impl<1, float, __half, true, true>(lv, gc, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials, O_PRE_LO_UPD, s);
     else if (P.precision == 2)
-        pre_impl<2, float, __nv_bfloat16, true, true>(g, gc, sm, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials,
+        pre_impl<2, float, __nv_bfloat16, true, true>(lv, gc, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials,
                                                       O_PRE_LO_UPD, s);
     else
-        pre_impl<0, float, float, true, true>(g, gc, sm, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials, O_PRE_F32_UPD,
+        pre_impl<0, float, float, true, true>(lv, gc, r_in, q, r_out, P.e0, P.lv[1].r, P.sc, partials, O_PRE_F32_UPD,
                                               s);
 }
 void mg_fused_post(const MGPlan& P, const float* r, double* partials, long long n_active, cudaStream_t s) {
-    const Grid3 &g = P.lv[0].L.g, &gc = P.lv[1].L.g;
-    const void* sm = P.lv[0].sm;
+    const MGLevel& lv = P.lv[0];
+    const Grid3& gc = P.lv[1].L.g;
     const void* ec1 = (1 < P.fused_levels) ? P.lv[1].eo : P.lv[1].e;
     if (P.precision == 1)
-        post_impl<1, float, __half, true, true>(g, gc, sm, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc, partials,
+        post_impl<1, float, __half, true, true>(lv, gc, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc, partials,
                                                 n_active, O_POST_LO, s);
     else if (P.precision == 2)
-        post_impl<2, float, __nv_bfloat16, true, true>(g, gc, sm, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc,
+        post_impl<2, float, __nv_bfloat16, true, true>(lv, gc, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc,
                                                        partials, n_active, O_POST_LO, s);
     else
-        post_impl<0, float, float, true, true>(g, gc, sm, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc, partials,
+        post_impl<0, float, float, true, true>(lv, gc, P.e0, ec1, r, P.lv[0].e, nullptr, P.prolong, P.sc, partials,
                                                n_active, O_POST_F32, s);
 }
 
-template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-static cudaError_t prep_pre(int kind) {
-    const void* fn = (const void*)k_presmooth_restrict<CK, VT, VTc, UPDATE, FINE>;
-    const size_t bytes = sizeof(PreRing<CK>);
+template <int CK>
+static cudaError_t prep_pass(const void* fn, size_t bytes, int kind) {
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess && kind >= 0) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f_occ[kind], fn, GeoOf<CK>::FT, bytes);
     return e;
 }
+template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
+static cudaError_t prep_pre(int kind) {
+    return prep_pass<CK>((const void*)k_presmooth_restrict<CK, VT, VTc, UPDATE, FINE>, sizeof(PreRing<CK>), kind);
+}
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
 static cudaError_t prep_post(int kind) {
-    const void* fn = (const void*)k_prolong_postsmooth<CK, VT, VTc, DOT, FINE>;
-    const size_t bytes = sizeof(PostRing<CK>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && kind >= 0) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f_occ[kind], fn, GeoOf<CK>::FT, bytes);
-    return e;
+    return prep_pass<CK>((const void*)k_prolong_postsmooth<CK, VT, VTc, DOT, FINE>, sizeof(PostRing<CK>), kind);
 }
 
 cudaError_t fused_prepare_attributes() {
@@ -868,6 +855,8 @@ cudaError_t fused_prepare_attributes() {
     PREP((prep_post<2, __nv_bfloat16, __nv_bfloat16, false, false>(-1)));
 #undef PREP
     if (e == cudaSuccess) e = tma_prepare_attributes();
+    if (e == cudaSuccess) e = run_prepare_attributes();
+    if (e == cudaSuccess) e = pair_prepare_attributes();
     return e;
 }
 

@@ -65,8 +65,10 @@ __device__ __forceinline__ Nbr neighbours(const Grid3& g, int x, int y, int z) {
 }
 
 // ------------------------------------------------------------- scalars
-__global__ void k_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, int max_total) {
+__global__ void k_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, double pass_margin,
+                               int max_total) {
     sc->tol2 = tol2;
+    sc->pass_margin = pass_margin;
     sc->max_total = max_total;
     sc->inv_sigma_z = 1.0f;
     sc->first = 1;
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_rhs(Grid3 g, int outlet, float
                 const bool done = !(bb > goal) || bb == 0.0;
                 sc->outer_done = done ? 1 : 0;
                 sc->converged = (done || !isfinite(bb)) ? 1 : 0;
-                sc->rr_target = fmax(sc->inner_floor2 * bb, 0.25 * goal);
+                sc->rr_target = fmax(sc->inner_floor2 * bb, sc->pass_margin * goal);
                 set_sigma_from(sc, bb, n_active);
                 sc->first = 1;
                 sc->alpha = sc->beta = 0.0;
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_residual(Grid3 g, const float4
             sc->outer_done = done ? 1 : 0;
             if (!isfinite(rr)) sc->nonfinite = 1;
             sc->converged = (done || !isfinite(rr)) ? 1 : 0;
-            sc->rr_target = fmax(sc->inner_floor2 * rr, 0.25 * goal);
+            sc->rr_target = fmax(sc->inner_floor2 * rr, sc->pass_margin * goal);
             set_sigma_from(sc, rr, n_active);
             // a new CG pass: the first search direction is z itself
             sc->first = 1;
@@ -1005,9 +1007,9 @@ void launch_coefficients(const Launch& L, const Fields& F, cudaStream_t s) {
     k_coefficients<<<L.grid, L.block, 0, s>>>(L.g, F.outlet, F.alpha, F.cls, F.mob, F.coef, F.coef_lo,
                                               F.coef_lo_kind, F.gtop);
 }
-void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, int max_total,
-                         cudaStream_t s) {
-    k_init_scalars<<<1, 1, 0, s>>>(sc, tol2, abs_floor, inner_floor2, max_total);
+void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, double pass_margin,
+                         int max_total, cudaStream_t s) {
+    k_init_scalars<<<1, 1, 0, s>>>(sc, tol2, abs_floor, inner_floor2, pass_margin, max_total);
 }
 void launch_set_sigma(Scalars* sc, float sigma, cudaStream_t s) { k_set_sigma<<<1, 1, 0, s>>>(sc, sigma); }
 // Measurement of the pipelined kernels in isolation: a mid-pass state with

@@ -34,7 +34,7 @@ struct Fields {
 
 // ---- GB300 solver kernels (gb300_kernels.cu)
 void launch_coefficients(const Launch& L, const Fields& F, cudaStream_t s);
-void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, int max_total,
+void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, double pass_margin, int max_total,
                          cudaStream_t s);
 // start_pass: also r = b, x = 0 and the first pass's scalars (a solve from x = 0)
 void launch_rhs(const Launch& L, const Fields& F, const float* u, const float* v, const float* w, cudaStream_t s,
@@ -93,7 +93,11 @@ struct MGLevel {
     void* r2;        // second-visit right-hand side of a fused W-cycle level (level precision)
     void* eo2;       // second-visit output of a fused W-cycle level (level precision)
     bool odd_periodic;
+    int passes;      // which fused passes a fused level runs (PASS_*)
 };
+// PASS_ASYNC: fused_kernels.cu (any grid); PASS_TMA: tma_fused.cu (its own
+// record layout); PASS_PAIR: tma_pair.cu; PASS_RUN: run_passes.cu.
+enum { PASS_ASYNC = 0, PASS_TMA, PASS_PAIR, PASS_RUN };
 // The levels of the bottom sub-cycle kernel (shared-memory offsets in floats
 // / float4s).
 struct BottomLevel {
@@ -136,6 +140,7 @@ struct MGPlan {
     int fused_levels;  // levels 0 .. fused_levels-1 run as fused pre-/post-smoothing passes (0: none)
     int bottom_from;   // levels from here down run in one bottom sub-cycle kernel (0: none)
     int w_from, w_to;  // levels w_from..w_to (>= 1) take two coarse visits, a W-cycle step (0: none)
+    long long w_min_bytes;  // finest-level records from which that step is taken
     bool w_disabled;   // the W-cycle step made the preconditioner indefinite here: V-cycles only
     size_t bottom_smem;
     BottomPlan bottom;
@@ -170,16 +175,37 @@ void launch_search_spmv(const Launch& L, const float4* coef, const float* z, con
 void launch_accumulate_pipelined(const Launch& L, float* x_hi, float* x_lo, const float* x, const float* p0,
                                  const float* p1, const Scalars* sc, cudaStream_t s);
 cudaError_t mg_prepare_attributes();
-// The same two passes with TMA-staged planes (tma_fused.cu), for grids without
-// periodic axes whose rows are whole 16-byte multiples; they return false, and
-// launch nothing, where they do not apply (the cp.async passes then run).
-// fine: level 0 (FP32 vectors, the level-precision coarse residual);
-// otherwise a coarse level in the level precision.
+// The two passes of a level without periodic axes whose x extent divides by
+// four, records staged by TMA (tma_fused.cu).  Such a level keeps its records
+// in their own layout (tma_records) and its pre-smoothed correction as the
+// compact black half.  fine: level 0 (FP32 vectors, the level-precision
+// coarse residual); otherwise a coarse level in the level precision.
 cudaError_t tma_prepare_attributes();
-bool tma_fused_enabled();
-bool tma_pre(int ck, bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin,
+bool tma_level_ok(const Grid3& g);
+size_t tma_record_bytes(const Grid3& g);
+bool tma_level_init(int ck, const Grid3& g, const void* sm);  // tma_level_ok and the copy map encodes
+void tma_records(int ck, const Launch& L, const void* coef, void* sm, cudaStream_t s);
+void tma_level_residual(int ck, const Launch& L, const void* sm, const void* r, const void* e, void* r2,
+                        const Scalars* sc, cudaStream_t s);
+void tma_pre(int ck, bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin,
              const float* q, float* r_out, void* e, void* rc, Scalars* sc, double* partials, cudaStream_t s);
-bool tma_post(int ck, bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
+void tma_post(int ck, bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
+              const void* r, void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active,
+              cudaStream_t s);
+
+// The passes of two half-steps of large FP32 levels (tma_pair.cu).
+cudaError_t pair_prepare_attributes();
+bool pair_level_init(const Grid3& g, const void* sm, const void* r);
+void pair_pre(bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q,
+              float* r_out, void* e, void* rc, Scalars* sc, double* partials, cudaStream_t s);
+void pair_post(bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r,
+               void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active, cudaStream_t s);
+// The passes of small levels, whole runs at once (run_passes.cu).
+cudaError_t run_prepare_attributes();
+bool run_level_ok(int ck, const Grid3& g);
+void run_pre(int ck, bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin,
+             const float* q, float* r_out, void* e, void* rc, Scalars* sc, double* partials, cudaStream_t s);
+void run_post(int ck, bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
               const void* r, void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active,
               cudaStream_t s);
 

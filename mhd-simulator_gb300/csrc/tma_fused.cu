@@ -1,946 +1,780 @@
-// tma_fused.cu -- the fused multigrid smoothing passes with planes staged by
-// the Tensor Memory Accelerator.
+// tma_fused.cu -- the multigrid smoothing passes of large levels with FP16 or
+// BF16 records, on grids without periodic axes: one pass down (residual update,
+// three half-steps from zero, restriction) and one pass up (prolongation, three
+// half-steps, the CG dot product), the smoother records staged by the Tensor
+// Memory Accelerator.
 //
-// k_pre_tma and k_post_tma do the work of k_presmooth_restrict and
-// k_prolong_postsmooth (fused_kernels.cu) with the same per-cell arithmetic
-// in the same order, so every vector they write is bit-identical; the
-// difference is how planes reach shared memory and how work is spread over
-// the threads:
+// Smoother.  A pass runs red, black, red half-steps of Gauss-Seidel, the
+// black one over-relaxed by SOR_BLACK:
+//   down, from zero:  e_r = r/d;  e_b = w (r + sum beta e_r)/d;
+//                     e_r += (sum beta e_b)/d
+//   up:               e_r = (r + sum beta e_b)/d;
+//                     e_b += w ((r + sum beta e_r)/d - e_b);
+//                     e_r = (r + sum beta e_b)/d
+// The up pass is the down pass reversed, so the cycle is symmetric.  Against
+// one red and one black half-step per pass the third one cuts the CG
+// iterations (jet 256^3: 22 -> 13, column 512x256x256: 14 -> 7, at an eighth of
+// the stopping residual) while the HBM traffic of a pass stays the same.  After
+// the down pass the residual is zero on red cells, so the restriction sums
+// black residuals only; the up pass overwrites the red values first, so only
+// the black half of the down pass's correction is kept in HBM (compact rows of
+// nx/2 values).
 //
-//  * One thread with no other task issues, per plane, one
-//    cp.async.bulk.tensor copy of each input: the smoother records (a 4-D box
-//    over the split rows: half-row columns, even/odd half, y, z), the level
-//    vectors (3-D boxes of RH rows from x0-4 for FP32 and from x0-8 for
-//    2-byte values, so the first coordinate stays 16-byte aligned) and, for
-//    the post-smoothing pass, the coarse correction (48 x CRH coarse cells
-//    from x0/2-8).  The copies of a plane complete on one mbarrier; two
-//    mbarriers alternate between planes.  Cells outside the grid arrive as
-//    zeros (the copy's out-of-bounds fill), which is the closed wall the
-//    cp.async zero fill stood for.  No thread computes a global address for a
-//    halo load, which removes most of the integer work of the cp.async
-//    kernels.
-//  * 384 threads (224 with FP32 records) take at most one task in every
-//    stage (360 red/prolongation quads, 324 black quads, 256 tile quads).
-//    The 16 interior quads of a staged row go to one half-warp, so its
-//    shared-memory accesses are contiguous; the halo quads of all rows follow.
-//  * Records and corrections sit in five-slot rings (planes zA-3 .. zA+1), so
-//    a step needs two barriers instead of three: warps that finish the tile
-//    stage of plane zA-2 go on to the next plane's red stage while others
-//    are still busy.
-
-// Only grids without periodic axes take these kernels (a copy box cannot
-// wrap around an axis); the cp.async kernels serve the others.  Every wait
-// on an mbarrier is bounded: when it runs out the block stops issuing
-// copies, marks the solve as stalled and converged (the host reports a
-// timeout), and finishes its loop without waiting again.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
+// Work split.  A block marches a 64 x FTY (x, y) tile along z.  A thread owns
+// one octet, eight consecutive cells of a row: the tile's octets and those of
+// the halo that some stage needs, ring by ring.  In an octet the cells of one
+// colour are the four cells of one x parity.  In step k a thread runs the
+// first half-step on plane k, the second on plane k-1, the third on plane k-2
+// and the output stage on plane k-3:
+//  * z neighbours are the thread's own values of the planes before and after,
+//    in registers;
+//  * x and y neighbours were written to shared memory by the previous step
+//    (two half-planes per stage, alternating), so a step has one barrier, and
+//    its stores come last so that the loads of the later stages overlap the
+//    arithmetic of the earlier ones;
+//  * the four cells a stage works on sit at the same x parity h in all of a
+//    step's planes, so the record half that a stage reads as its own holds
+//    the z-high mobilities of the next stage: they pass on in registers;
+//  * the steps of the two parities are straight-line code, one copy for the
+//    warps with the tile's octets and one for the halo's.
+// What bounds it: the latency of a step (about 2200 cycles: the stages' shared
+// memory loads and dependent sums, twelve warps per SM) and the L2 traffic of
+// the halo (1.5 reads per cell).  jet 256^3, FP16 records: 121 us down, 120 us
+// up (400 and 335 MB of HBM traffic).  Passes of two half-steps on quads with
+// every neighbour from shared memory took 101 and 98 us; three half-steps in
+// that form would take half as long again.  16 tile rows and two blocks per
+// SM: 142 and 154 us (halo 1.7, registers capped at 128); values of earlier
+// planes from shared memory instead of registers: 152 and 192 us.
+//
+// Records in HBM: per grid row four half rows of `pitch` entries: (beta_x,
+// beta_y) of the even-x cells, of the odd-x cells, (beta_z, diagonal) of the
+// even-x cells, of the odd-x cells; an entry is two FP16/BF16 values.  Rows are
+// padded to 16 bytes.  One cp.async.bulk.tensor box of 40 entries x 4 half
+// rows x RH rows brings a plane (entries x0/2-4 .. x0/2+35: the first
+// coordinate is 16-byte aligned); cells outside the grid arrive as zeros, the closed wall.
+//
+// Every wait on an mbarrier is bounded: when it runs out the block stops
+// issuing copies, marks the solve as stalled and converged (the host reports
+// a timeout), and finishes its loop without waiting again.  Periodic grids
+// (a copy box cannot wrap around) take the passes of fused_kernels.cu.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <mutex>
 
 #include "kernels.h"
 #include "fused_common.cuh"
+#include "tma_common.cuh"
 
 namespace mhdproj {
 
 namespace {
 using namespace staged;
 using namespace fused;
+using namespace tma;
+
+constexpr int HH = 40;         // staged entries of a half row: x0/2-4 .. x0/2+35
+constexpr int NO = 10;         // octets of a staged row: x0-8 .. x0+71
+constexpr int QO = PX / 8;     // own octets of a row
+constexpr int RS = 4 * HH;     // entries of a staged record row
 
 template <int CK>
-struct TGeo {
-    static constexpr int FTY = CK == 0 ? 8 : 16;       // tile rows
-    static constexpr int RH = FTY + 4;                 // staged rows y0-2 .. y0+FTY+1
-    static constexpr int NRED = RH * NQ;               // red / prolongation quads
-    static constexpr int NBR = FTY + 2;                // black rows y0-1 .. y0+FTY
-    static constexpr int NBLK = NBR * NQ;              // black quads
-    static constexpr int NOWN = QX * FTY;              // tile quads
-    static constexpr int NT = (NRED + 32) / 32 * 32;   // threads: one red task each, and a spare issuing thread
-    static constexpr int CRH = FTY / 2 + 2;            // coarse rows y0/2-1 .. y0/2+FTY/2
-    static constexpr int CW = 48;                      // coarse columns x0/2-8 .. x0/2+39
-    static constexpr int NS = 5;                       // ring slots of records and corrections: zA-3 .. zA+1
-    static constexpr int NP = 6;                       // planes of a run of two with its halo (whole-run passes)
-    static_assert(NBLK <= NT && NOWN <= NT && NRED < NT, "one task per thread");
+struct OGeo {
+    static constexpr int FTY = 32;                     // tile rows
+    static constexpr int RH = FTY + 6;                 // staged rows y0-3 .. y0+FTY+2
+    static constexpr int C0 = QO * FTY / 2;            // own octets of one row parity
+    static constexpr int WP = C0 / 32 + 2;             // warps per row parity: own octets, then the halo's
+    static constexpr int NT = 64 * WP;                 // threads; the last one only issues copies
+    static constexpr int NS = 5;                       // record ring: planes k+1 .. k-3
+    static_assert(C0 % 32 == 0, "own octets fill warps");
 };
-// Staged rows of a level vector: x0-4 .. x0+67 for FP32 (the first
-// coordinate x0-4 is 16-byte aligned), x0-8 .. x0+71 for 2-byte values.
-template <class VT>
-struct VGeo {
-    static constexpr int XS = sizeof(VT) == 4 ? 4 : 8;  // row starts at x0 - XS
-    static constexpr int VW = sizeof(VT) == 4 ? 72 : 80;
-    static constexpr int VX = XS - XO;                 // column of x0-4 in a staged row
-};
-constexpr int TMA_MIN_BLOCKS = 2;
-constexpr int WAIT_LIMIT = 1 << 22;
-
-// ------------------------------------------------------------- PTX wrappers
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(b)), "r"(count) : "memory");
+// Record entries: two values.
+using Entry = unsigned;
+// Four entries of a half row as loaded.
+template <int CK> struct Rec4 { uint4 v; };
+template <int CK>
+__device__ __forceinline__ Rec4<CK> ld_rec(const Entry* p) {
+    return Rec4<CK>{*reinterpret_cast<const uint4*>(p)};
 }
-__device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
-// Orders this thread's (and, after a barrier, the block's) generic-proxy
-// accesses of shared memory before the copies it issues next.
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+template <int CK>
+__device__ __forceinline__ float half_lo(unsigned u) {
+    if constexpr (CK == 1) return __low2float(*reinterpret_cast<const __half2*>(&u));
+    else return __uint_as_float(u << 16);
 }
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(b)), "r"(parity)
-        : "memory");
-    return ok != 0;
+template <int CK>
+__device__ __forceinline__ float half_hi(unsigned u) {
+    if constexpr (CK == 1) return __high2float(*reinterpret_cast<const __half2*>(&u));
+    else return __uint_as_float(u & 0xffff0000u);
 }
-// Bounded wait for the phase of the given parity; false when it ran out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
-    for (int i = 0; i < WAIT_LIMIT; i++)
-        if (mbar_try_wait(b, parity)) return true;
-    return false;
+// The first / second values of the four entries.
+template <int CK>
+__device__ __forceinline__ void rec_lo(const Rec4<CK>& r, float (&o)[4]) {
+    o[0] = half_lo<CK>(r.v.x); o[1] = half_lo<CK>(r.v.y); o[2] = half_lo<CK>(r.v.z); o[3] = half_lo<CK>(r.v.w);
 }
-__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* tm, int x, int y, int z, unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];\n" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<unsigned long long>(tm)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tma_4d(void* dst, const CUtensorMap* tm, int x, int h, int y, int z,
-                                       unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-        "%5}], [%6];\n" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<unsigned long long>(tm)), "r"(x), "r"(h), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
+template <int CK>
+__device__ __forceinline__ void rec_hi(const Rec4<CK>& r, float (&o)[4]) {
+    o[0] = half_hi<CK>(r.v.x); o[1] = half_hi<CK>(r.v.y); o[2] = half_hi<CK>(r.v.z); o[3] = half_hi<CK>(r.v.w);
 }
 
-template <class T, int N>
-constexpr int padded128() {  // elements of N T rounded up to 128 bytes
-    return (int)(((N * sizeof(T) + 127) / 128) * 128 / sizeof(T));
-}
-
-// Shared memory of the pre-smoothing pass: records and corrections of planes
-// zA-3 .. zA+1 (five slots), the copied residual and q of planes zA, zA+1.
-template <int CK, class VT, bool UPDATE>
-struct PreTmaSm {
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    using VQ = VGeo<float>;
-    alignas(128) CT c[G::NS][G::RH][RW];
-    alignas(128) VT rv[2][G::RH][V::VW];
-    alignas(128) float qv[UPDATE ? 2 : 1][UPDATE ? G::RH : 1][VQ::VW];
-    alignas(16) float er[G::NS][G::RH][RW];
-    float2 ypart[G::FTY][QX];
+template <int CK>
+struct PassSm {
+    using ET = Entry;
+    using G = OGeo<CK>;
+    alignas(128) ET c[G::NS][G::RH][RS];
+    // the three stages' half-planes, each for the next step (slot: step & 1)
+    alignas(16) float ex[3][2][G::RH][HH];
+    float4 ypart[G::FTY / 2][QO];  // restriction sums of the odd rows
     unsigned long long bar[2];
     int abort_;
 };
-// Shared memory of the post-smoothing pass: records and smoothed corrections
-// of planes zA-3 .. zA+1, the copied pre-smoothed correction and right-hand
-// side of planes zA, zA+1, and the coarse correction of the two coarse
-// planes they fall in.
-template <int CK, class VT, class VTc>
-struct PostTmaSm {
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    static constexpr int ECS = padded128<VTc, G::CRH * G::CW>();
-    alignas(128) CT c[G::NS][G::RH][RW];
-    alignas(128) VT ev[2][G::RH][V::VW];
-    alignas(128) VT rv[2][G::RH][V::VW];
-    alignas(128) VTc ec[2][ECS];
-    alignas(16) float ep[G::NS][G::RH][RW];
-    unsigned long long bar[2];
-    int abort_;
+
+// A thread's octet: staged row, octet in the row, halo ring (0: own, 4: none).
+// The rows of a warp have one parity, so the colour of a half row is the same
+// for all its lanes, and the warps of the two parities alternate, so that the
+// warps with own octets (the most stages) spread over the four schedulers.
+// The rings follow the seven-point stencil: a ring's corners belong to the
+// next one.  Record rows start at the same bank, so the halo's octets are
+// dealt out over groups of eight lanes (the lanes that load together): the
+// side octets of two rows, then octets of the rows beyond the tile.
+__device__ __forceinline__ int octet_index(int t) { return (t >> 6) * 32 + (t & 31); }
+template <class G>
+struct Octet {
+    int row, oc, ring;
+    __device__ __forceinline__ explicit Octet(int t) {
+        constexpr int RPG = G::FTY >= 16 ? G::FTY / 16 : 1;  // rows whose sides one group holds
+        const int par = (t >> 5) & 1, u = octet_index(t);
+        int ty = par;
+        oc = 1;
+        ring = 4;
+        if (u < G::C0) {
+            ty = 2 * (u / QO) + par;
+            oc = 1 + u % QO;
+            ring = 0;
+        } else {
+            const int e = u - G::C0, grp = e >> 3, j = e & 7;
+            if (j < 2 * RPG) {
+                const int rr = grp * RPG + (j >> 1);
+                if (rr < G::FTY / 2) {
+                    ty = 2 * rr + par;
+                    oc = (j & 1) ? NO - 1 : 0;
+                    ring = 1;
+                }
+            } else {
+                // rows beyond the tile, eight octets each: -1 / FTY (ring 1), -2 / FTY+1
+                // (ring 2), -3 / FTY+2 (ring 3); corners of the first (ring 2) and of
+                // the second (ring 3)
+                const int m = grp * (8 - 2 * RPG) + (j - 2 * RPG);
+                int out = 0;
+                if (m < 3 * QO) {
+                    out = ring = 1 + m / QO;
+                    oc = 1 + m % QO;
+                } else if (m < 3 * QO + 4) {
+                    const int c = m - 3 * QO;
+                    out = 1 + (c >> 1);
+                    ring = out + 1;
+                    oc = (c & 1) ? NO - 1 : 0;
+                }
+                if (out) {
+                    const bool low = ((out & 1) != 0) == (par != 0);
+                    ty = low ? -out : G::FTY - 1 + out;
+                }
+            }
+        }
+        row = ty + 3;
+    }
 };
-template <class SM>
-__device__ __forceinline__ SM& aligned_smem(unsigned char* raw) {
-    return *reinterpret_cast<SM*>(raw + ((128u - (smem_u32(raw) & 127u)) & 127u));
+
+// 1/d for a positive diagonal, 0 for a cell without one.
+__device__ __forceinline__ float rcp_or_zero(float d) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return d > 1e-37f ? r : 0.0f;
+}
+__device__ __forceinline__ void put4(float* p, const float (&v)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void copy4(float (&a)[4], const float (&b)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) a[j] = b[j];
 }
 
-// Task of thread t in a stage over `rows` staged rows starting at row0: the
-// 16 interior quads (1 .. 16) of a row go to one half-warp, so its
-// shared-memory accesses are contiguous and free of bank conflicts; the two
-// halo quads of each row (0 and 17) follow as tasks rows*16 .. rows*18-1.
-__device__ __forceinline__ void stage_task(int t, int rows, int row0, int* row, int* q) {
-    if (t < rows * 16) {
-        *row = row0 + (t >> 4);
-        *q = 1 + (t & 15);
-    } else {
-        const int e = t - rows * 16;
-        *row = row0 + (e >> 1);
-        *q = (e & 1) ? NQ - 1 : 0;
+__device__ __forceinline__ void get4(float (&v)[4], const float* p) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+    v[2] = t.z;
+    v[3] = t.w;
+}
+// beta_x of one entry.
+template <int CK>
+__device__ __forceinline__ float entry_lo(const Entry* p) {
+    return half_lo<CK>(*p);
+}
+// Sums of beta times the other colour over the six neighbours of an octet's
+// four cells of x parity H, added to acc; d: their diagonals; bz: in, the
+// z-high mobilities (of plane + 1), out, their own z-low ones (the z-high
+// ones of the stage one plane below).  C: the octet's first entry in its
+// record plane; X: the other colour's half-plane at the octet; o, zm, zp: the
+// octet's values of the other colour in this plane, the one below and the
+// one above.  At the ends of a staged row the outermost cell takes a value of
+// another row: nothing reads that cell.
+template <int CK, int H>
+__device__ __forceinline__ void gs_octet(const Entry* C, const float* X, const float (&o)[4],
+                                         const float (&zm)[4], const float (&zp)[4], float (&bz)[4], float (&acc)[4],
+                                         float (&d)[4]) {
+    const Rec4<CK> A = ld_rec<CK>(C + H * HH), Q = ld_rec<CK>(C + (1 - H) * HH);
+    const Rec4<CK> Y = ld_rec<CK>(C + RS + H * HH), B = ld_rec<CK>(C + (2 + H) * HH);
+    float m[4], p[4];
+    get4(m, X - HH);
+    get4(p, X + HH);
+    const float s = X[H ? 4 : -1];
+    const float a4 = H ? entry_lo<CK>(C + 4) : 0.f;
+    float bxl[4], byl[4], byh[4], t[4], bzl[4];
+    rec_lo<CK>(A, bxl);
+    rec_hi<CK>(A, byl);
+    rec_hi<CK>(Y, byh);
+    rec_lo<CK>(B, bzl);
+    rec_hi<CK>(B, d);
+    rec_lo<CK>(Q, t);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float left = H ? o[j] : (j ? o[j - 1] : s), right = H ? (j < 3 ? o[j + 1] : s) : o[j];
+        const float bxh = H ? (j < 3 ? t[j + 1] : a4) : t[j];
+        float a = acc[j];
+        a = fmaf(bxl[j], left, a);
+        a = fmaf(bxh, right, a);
+        a = fmaf(byl[j], m[j], a);
+        a = fmaf(byh[j], p[j], a);
+        a = fmaf(bzl[j], zm[j], a);
+        a = fmaf(bz[j], zp[j], a);
+        acc[j] = a;
+        bz[j] = bzl[j];
     }
 }
+__device__ __forceinline__ void block_bar() { asm volatile("bar.sync 0;\n" ::: "memory"); }
 
-// ------------------------------------------------------ pre-smoothing pass
-// See k_presmooth_restrict for the algebra; rin and q arrive through tm_r
-// and tm_q, the records through tm_rec.  A step handles the red stage of
-// plane zA, the black stage of zA-1 and the tile stage of zA-2 with two
-// barriers: the five-slot rings let the next step's copies and red stage
-// start while other warps still finish the tile stage.
+// The plane ring of records: issue, wait and slot bookkeeping shared by the
+// two passes.
+template <int CK>
+struct RecordRing {
+    using G = OGeo<CK>;
+    using SM = PassSm<CK>;
+    static constexpr int ISSUER = G::NT - 1;
+    static constexpr unsigned BYTES = G::RH * RS * sizeof(Entry);
+    SM& S;
+    const CUtensorMap* tm;
+    int x0, y0, zs, last = 0;
+    static constexpr int SLOT = G::RH * RS;
+    // ring offsets of planes k .. k-3 and of the next copy's slot
+    int s0 = 0, s1 = (G::NS - 1) * SLOT, s2 = (G::NS - 2) * SLOT, s3 = (G::NS - 3) * SLOT, ahead = SLOT;
+    __device__ __forceinline__ RecordRing(SM& S_, const CUtensorMap* tm_, int x0_, int y0_, int zs_)
+        : S(S_), tm(tm_), x0(x0_), y0(y0_), zs(zs_) {
+        if (threadIdx.x == ISSUER) {
+            mbar_init(&S.bar[0], 1);
+            mbar_init(&S.bar[1], 1);
+            S.abort_ = 0;
+            fence_barrier_init();
+        }
+        __syncthreads();
+        if (threadIdx.x == ISSUER) issue(0, 0);
+    }
+    __device__ __forceinline__ void issue(int k, int off) {  // the copy of plane zs + k (ring offset off)
+        unsigned long long* b = &S.bar[k & 1];
+        fence_proxy_async();
+        mbar_expect_tx(b, BYTES);
+        tma_4d(&S.c[0][0][0] + off, tm, (x0 >> 1) - 4, 0, y0 - 3, zs + k, b);
+        last = k;
+    }
+    // step k: rotate the slots, issue plane k+1 into the slot of plane k-4, wait
+    // for plane k
+    __device__ __forceinline__ void step(int k, int nsteps, Scalars* sc) {
+        if (k) {
+            const int t = s3;
+            s3 = s2;
+            s2 = s1;
+            s1 = s0;
+            s0 = ahead;
+            ahead = t;
+        }
+        const bool aborted = *reinterpret_cast<volatile int*>(&S.abort_) != 0;
+        if (threadIdx.x == ISSUER && k + 1 < nsteps && !aborted) issue(k + 1, ahead);
+        if (!aborted && !mbar_wait(&S.bar[k & 1], (k >> 1) & 1)) {
+            S.abort_ = 1;
+            sc->stalled = 1;
+            sc->converged = 1;
+        }
+    }
+    // after a timed-out wait the copies in flight land before the block exits
+    __device__ __forceinline__ void drain() {
+        if (threadIdx.x == ISSUER && S.abort_)
+            for (int j = max(0, last - 1); j <= last; j++) (void)mbar_wait(&S.bar[j & 1], (j >> 1) & 1);
+    }
+};
+
+// ---------------------------------------------------------------- down pass
+// rin (VT) -> the black half of the correction (compact rows) and the coarse
+// residual rc.  UPDATE (finest level inside CG): r_out = rin - alpha q is
+// formed first, written for the tile's cells, and ||r_out||^2 decides
+// convergence.  FINE: the right-hand side is sigma * r.
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-__global__ void __launch_bounds__(TGeo<CK>::NT, TMA_MIN_BLOCKS)
-    k_pre_tma(const __grid_constant__ CUtensorMap tm_rec, const __grid_constant__ CUtensorMap tm_r,
-              const __grid_constant__ CUtensorMap tm_q, Grid3 g, Grid3 gc, float* __restrict__ r_out,
-              VT* __restrict__ e, VTc* __restrict__ rc, Scalars* sc, double* partials, int nblocks) {
+__global__ void __launch_bounds__(OGeo<CK>::NT, 1)
+    k_pre_tma(const __grid_constant__ CUtensorMap tm_rec, Grid3 g, Grid3 gc, const VT* __restrict__ rin,
+              const float* __restrict__ q, float* __restrict__ r_out, VT* __restrict__ ek, VTc* __restrict__ rc,
+              Scalars* sc, double* partials, int nblocks) {
     if (sc->converged) return;
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    using VQ = VGeo<float>;
-    using SM = PreTmaSm<CK, VT, UPDATE>;
+    using ET = Entry;
+    using G = OGeo<CK>;
+    using SM = PassSm<CK>;
     using R4 = typename Raw4<VT>::T;
-    constexpr int FTY = G::FTY, NT = G::NT, RH = G::RH, NS = G::NS, SL = RH * RW;
-    constexpr unsigned BYTES =
-        RH * RW * sizeof(CT) + RH * V::VW * sizeof(VT) + (UPDATE ? RH * VQ::VW * 4 : 0);
+    constexpr int NT = G::NT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SM& S = aligned_smem<SM>(smem_raw);
     __shared__ double sh[NT / 32];
     const int t = threadIdx.x;
-    constexpr int ISSUER = NT - 1;  // no task in any stage
     const float sigma = FINE ? sc->sigma : 1.0f;
     const float alpha = UPDATE ? sc->alpha_f : 0.0f;
-    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * FTY;
+    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * G::FTY;
     const int z0 = blockIdx.z * g.zper, z1 = min(g.nz, z0 + g.zper);
-    const int zs = z0 - 2, nsteps = z1 - z0 + 4;  // planes zs .. z1+1
-    const long long sxy = (long long)g.nx * g.ny;
-    int last_issued = 0;
-    auto issue = [&](int k, int off) {  // the copies of plane zs + k
-        const int zz = zs + k;
-        unsigned long long* b = &S.bar[k & 1];
-        fence_proxy_async();
-        mbar_expect_tx(b, BYTES);
-        tma_4d(&S.c[0][0][0] + off, &tm_rec, 2 * x0 - 8, 0, y0 - 2, zz, b);
-        tma_3d(&S.rv[k & 1][0][0], &tm_r, x0 - V::XS, y0 - 2, zz, b);
-        if (UPDATE) tma_3d(&S.qv[k & 1][0][0], &tm_q, x0 - VQ::XS, y0 - 2, zz, b);
-        last_issued = k;
+    const int zs = z0 - 3, nsteps = z1 - z0 + 6;  // planes zs .. z1+2
+    const Octet<G> T(t);
+    const int gx = x0 - 8 + 8 * T.oc, gy = y0 - 3 + T.row;
+    const bool in_y = T.ring < 4 && gy >= 0 && gy < g.ny;
+    // of the side octets only the quad next to the tile is read
+    const bool in_a = in_y && T.oc != 0 && gx < g.nx, in_b = in_y && T.oc != NO - 1 && gx + 4 >= 0 && gx + 4 < g.nx;
+    const bool own_warp = octet_index(t) < G::C0;
+    const int sxy = g.nx * g.ny, go = gx + g.nx * gy;
+    // rows 0 and RH-1 run no stage that reads their outer rows; lanes off a
+    // stage read in range and are not stored
+    const int rs = min(max(T.row, 1), G::RH - 2);
+    const ET* const c_own = &S.c[0][rs][4 * T.oc];
+    const ET* const c_r0 = &S.c[0][T.row][4 * T.oc];
+    float* const x_own = &S.ex[0][0][rs][4 * T.oc];
+    float* const x_put = &S.ex[0][0][T.row][4 * T.oc];
+    constexpr int XP = G::RH * HH, ST = 2 * XP;  // one half-plane, one stage
+    R4 rv[2];
+    float4 qv[2];
+    auto load = [&](int zz) {  // the octet's residual (and q) of plane zz
+        const bool okz = zz >= 0 && zz < g.nz;  // (planes beyond the last one are loaded and not used)
+        const long long o = (long long)sxy * zz + go;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const bool ok = okz && (u ? in_b : in_a);
+            rv[u] = ldg_quad<VT>(rin + o + 4 * u, ok);
+            if (UPDATE) qv[u] = ldg_quad<float>(q + o + 4 * u, ok);
+        }
     };
-    if (t == ISSUER) {
-        mbar_init(&S.bar[0], 1);
-        mbar_init(&S.bar[1], 1);
-        S.abort_ = 0;
-        fence_barrier_init();
-    }
-    __syncthreads();
-    if (t == ISSUER) issue(0, 0);
-
-    // red task
-    int r_row, r_q;
-    stage_task(t, RH, 0, &r_row, &r_q);
-    const bool has_red = t < G::NRED;
-    const int r_o = r_row * RW + 2 * r_q;             // split offset of the quad's even half
-    const int r_v = r_row * V::VW + V::VX + 4 * r_q;  // its cells in a copied vector row
-    const int r_qv = r_row * VQ::VW + VQ::VX + 4 * r_q;
-    const int r_gx = x0 - XO + 4 * r_q, r_gy = y0 - 2 + r_row;
-    const int r_par = r_gy & 1;
-    const int r_own = (has_red && r_row >= 2 && r_row < FTY + 2 && r_q >= 1 && r_q <= QX && r_gx < g.nx && r_gy < g.ny)
-                          ? r_gx + g.nx * r_gy
-                          : -1;
-    // black task
-    int b_row, b_q;
-    stage_task(t, G::NBR, 1, &b_row, &b_q);
-    const bool has_blk = t < G::NBLK;
-    const int b_o = b_row * RW + 2 * b_q;
-    const int b_par = (y0 - 2 + b_row) & 1;
-    // tile task: the own quad
-    const bool has_own = t < G::NOWN;
-    const int tx = t % QX, ty = t / QX;
-    const int ox = x0 + 4 * tx, oy = y0 + ty;
-    const bool own_inside = has_own && ox < g.nx && oy < g.ny;
-    const int oo = (ty + 2) * RW + 2 * (tx + 1);
-    const long long og = ox + (long long)g.nx * oy;
-
-    const CT* c0 = &S.c[0][0][0];
-    float* e0 = &S.er[0][0][0];
+    load(zs);
+    RecordRing<CK> ring(S, &tm_rec, x0, y0, zs);
     float rr_thread = 0.f;
-    float2 part = make_float2(0.f, 0.f);
-    int rc_z = -1;
+    // restriction sums of the coarse planes of planes k-3 and k-1; the finished
+    // ones of the even rows until the odd rows' arrive
+    float pa[4] = {}, pb[4] = {}, ph[4] = {};
+    int rc_z = -1;  // coarse plane of ph
     auto flush_rc = [&]() {
-        if (rc_z >= 0 && own_inside && !(ty & 1)) {
-            const float2 a = S.ypart[ty][tx], b = S.ypart[ty + 1][tx];
-            st2<VTc>(rc + (ox >> 1) + (long long)gc.nx * ((oy >> 1) + (long long)gc.ny * rc_z),
-                     make_float2(0.25f * (a.x + b.x), 0.25f * (a.y + b.y)));
+        if (rc_z >= 0 && own_warp && !(gy & 1)) {
+            const float4 o = S.ypart[(T.row - 3) >> 1][T.oc - 1];
+            VTc* cp = rc + ((gx >> 1) + (long long)gc.nx * ((gy >> 1) + (long long)gc.ny * rc_z));
+            if (in_a) st2<VTc>(cp, make_float2(0.25f * (ph[0] + o.x), 0.25f * (ph[1] + o.y)));
+            if (in_b) st2<VTc>(cp + 2, make_float2(0.25f * (ph[2] + o.z), 0.25f * (ph[3] + o.w)));
         }
         rc_z = -1;
     };
-    // element offsets of the ring slots of planes zA, zA-1, zA-2, zA-3
-    int o0 = 0, o1 = (NS - 1) * SL, o2 = (NS - 2) * SL, o3 = (NS - 3) * SL;
-    auto step = [&](auto ph, int k) {
-        constexpr int P = decltype(ph)::value;  // k & 3; zs is even, so plane zA has parity P & 1
+    // the octet's values by step parity: first-stage reds (index H: plane k-2,
+    // 1-H: k-1), blacks (H: k-2, 1-H: k-3), third-stage reds (H: k-4, 1-H: k-3);
+    // black right-hand side of plane k-1
+    float r_[2][4] = {}, b_[2][4] = {}, f_[2][4] = {}, g1[4] = {};
+    auto step = [&](auto hc, auto role, int k) {
+        constexpr int H = decltype(hc)::value;  // red half of plane k, black half of plane k-1, ...
+        constexpr int ROLE = decltype(role)::value;
         const int zA = zs + k;
-        const bool aborted = *reinterpret_cast<volatile int*>(&S.abort_) != 0;
-        if (t == ISSUER && k + 1 < nsteps && !aborted) issue(k + 1, o0 == (NS - 1) * SL ? 0 : o0 + SL);
-        if (!aborted && !mbar_wait(&S.bar[P & 1], P >> 1)) {
-            S.abort_ = 1;
-            sc->stalled = 1;
-            sc->converged = 1;
-        }
-        // ---- red stage: plane zA over the 2-halo rows
-        if (has_red) {
-            const CT* C = c0 + o0;
-            float* ER = e0 + o0;
-            float4 rn = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.rv[P & 1][0][0] + r_v));
+        const int cur = (k & 1) * XP, prv = XP - cur;
+        ring.step(k, nsteps, sc);
+        if (ROLE == 0) flush_rc();
+        // ---- first red half-step, plane k
+        float r0[4], g0[4], bz[4];
+        {
+            float4 ra = cvt4r<VT>(rv[0]), rb = cvt4r<VT>(rv[1]);
             if (UPDATE) {
-                const float4 qq = *reinterpret_cast<const float4*>(&S.qv[P & 1][0][0] + r_qv);
-                rn = make_float4(fmaf(-alpha, qq.x, rn.x), fmaf(-alpha, qq.y, rn.y), fmaf(-alpha, qq.z, rn.z),
-                                 fmaf(-alpha, qq.w, rn.w));
-            }
-            const int p = r_par ^ (P & 1);
-            float4 d0, d1;
-            rec2<CK>(C + r_o + p * HW, &d0, &d1);
-            const float2 rr = p ? make_float2(rn.y, rn.w) : make_float2(rn.x, rn.z);  // red cells
-            const float2 rb = p ? make_float2(rn.x, rn.z) : make_float2(rn.y, rn.w);  // black cells
-            const float2 ev = divide2(make_float2(sigma * rr.x, sigma * rr.y), make_float2(d0.w, d1.w));
-            *reinterpret_cast<float2*>(ER + r_o + p * HW) = ev;
-            *reinterpret_cast<float2*>(ER + r_o + (1 - p) * HW) = make_float2(sigma * rb.x, sigma * rb.y);
-            if (UPDATE && r_own >= 0 && zA >= z0 && zA < z1) {
-                *reinterpret_cast<float4*>(r_out + sxy * zA + r_own) = rn;
-                rr_thread = fmaf(rn.x, rn.x, fmaf(rn.y, rn.y, fmaf(rn.z, rn.z, fmaf(rn.w, rn.w, rr_thread))));
-            }
-        }
-        __syncthreads();
-        flush_rc();
-        // ---- black stage: plane zA-1 over the 1-halo rows, in place
-        if (has_blk && zA - 1 >= z0 - 1) {
-            const CT* C = c0 + o1;
-            const CT* CN = c0 + o0;
-            float* E = e0 + o1;
-            const float* EM = e0 + o2;
-            const float* EP = e0 + o0;
-            const int h = b_par ^ (P & 1);  // black half of the row at plane zA-1
-            const int o = b_o + h * HW;
-            float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, o, h, *reinterpret_cast<const float2*>(E + o), &d);
-            *reinterpret_cast<float2*>(E + o) = divide2(s, d);
-        }
-        __syncthreads();
-        // ---- correction out and restriction: plane zA-2 over the tile
-        const int zC = zA - 2;
-        if (has_own && zC >= z0 && zC < z1) {
-            const CT* C = c0 + o2;
-            const CT* CN = c0 + o1;
-            const float* E = e0 + o2;
-            const float* EM = e0 + o3;
-            const float* EP = e0 + o1;
-            const int p = (oy & 1) ^ (P & 1);  // red half of the own quad
-            float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, oo + p * HW, p, make_float2(0.f, 0.f), &d);
-            part.x += s.x;
-            part.y += s.y;
-            if (own_inside) {
-                const float2 ev = *reinterpret_cast<const float2*>(E + oo);
-                const float2 od = *reinterpret_cast<const float2*>(E + oo + HW);
-                st4<VT>(e + (og + sxy * zC), make_float4(ev.x, od.x, ev.y, od.y));
-            }
-            if ((zC & 1) || zC + 1 == z1) {
-                // the row pair sum is formed after the next step's first barrier
-                S.ypart[ty][tx] = part;
-                rc_z = zC >> 1;
-                part = make_float2(0.f, 0.f);
-            }
-        }
-    };
-    auto advance = [&]() {
-        o3 = o2;
-        o2 = o1;
-        o1 = o0;
-        o0 = o0 == (NS - 1) * SL ? 0 : o0 + SL;
-    };
-    for (int k = 0;;) {
-        step(Phase<0>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<1>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<2>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<3>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-    }
-    __syncthreads();
-    flush_rc();
-    if (t == ISSUER && S.abort_) (void)mbar_wait(&S.bar[last_issued & 1], (last_issued >> 1) & 1);
-    if (UPDATE) {
-        double v1[1] = {(double)rr_thread};
-        block_sum<1>(v1, sh);
-        if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[8])) {
-            double tot[1];
-            finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[8]);
-            if (t == 0 && !sc->stalled) {
-                const double rr = tot[0];
-                sc->rr = rr;
-                sc->iterations += 1;
-                sc->total_iterations += 1;
-                if (!isfinite(rr)) {
-                    sc->nonfinite = 1;
-                    sc->converged = 1;
-                } else if (rr <= sc->rr_target || sc->total_iterations >= sc->max_total) {
-                    sc->converged = 1;
+                ra = make_float4(fmaf(-alpha, qv[0].x, ra.x), fmaf(-alpha, qv[0].y, ra.y), fmaf(-alpha, qv[0].z, ra.z),
+                                 fmaf(-alpha, qv[0].w, ra.w));
+                rb = make_float4(fmaf(-alpha, qv[1].x, rb.x), fmaf(-alpha, qv[1].y, rb.y), fmaf(-alpha, qv[1].z, rb.z),
+                                 fmaf(-alpha, qv[1].w, rb.w));
+                if (ROLE == 0 && zA >= z0 && zA < z1) {
+                    float* rp = r_out + ((long long)sxy * zA + go);
+                    if (in_a) *reinterpret_cast<float4*>(rp) = ra;
+                    if (in_b) *reinterpret_cast<float4*>(rp + 4) = rb;
+                    rr_thread = fmaf(ra.x, ra.x, fmaf(ra.y, ra.y, fmaf(ra.z, ra.z, fmaf(ra.w, ra.w, rr_thread))));
+                    rr_thread = fmaf(rb.x, rb.x, fmaf(rb.y, rb.y, fmaf(rb.z, rb.z, fmaf(rb.w, rb.w, rr_thread))));
                 }
             }
+            load(zA + 1);
+            const Rec4<CK> B = ld_rec<CK>(c_r0 + ring.s0 + (2 + H) * HH);
+            float d[4];
+            rec_lo<CK>(B, bz);
+            rec_hi<CK>(B, d);
+            const float re[4] = {ra.x, ra.z, rb.x, rb.z}, rd[4] = {ra.y, ra.w, rb.y, rb.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                r0[j] = (H ? rd[j] : re[j]) * (sigma * rcp_or_zero(d[j]));
+                g0[j] = sigma * (H ? re[j] : rd[j]);
+            }
         }
-    }
+        // ---- black half-step, plane k-1
+        float b1[4], f2[4], acc[4], d[4];
+        copy4(acc, g1);
+        gs_octet<CK, H>(c_own + ring.s1, x_own + prv, r_[1 - H], r_[H], r0, bz, acc, d);
+#pragma unroll
+        for (int j = 0; j < 4; j++) b1[j] = acc[j] * (SOR_BLACK * rcp_or_zero(d[j]));
+        if (ROLE == 0 && k >= 4) {  // right-hand side minus d e of the black residual
+#pragma unroll
+            for (int j = 0; j < 4; j++) pb[j] += fmaf(-d[j], b1[j], g1[j]);
+        }
+        copy4(g1, g0);
+        // ---- second red half-step, plane k-2
+        if constexpr (ROLE <= 1) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[j] = 0.f;
+            gs_octet<CK, H>(c_own + ring.s2, x_own + ST + prv, b_[H], b_[1 - H], b1, bz, acc, d);
+#pragma unroll
+            for (int j = 0; j < 4; j++) f2[j] = fmaf(acc[j], rcp_or_zero(d[j]), r_[H][j]);
+            // ---- correction out, black residual and restriction, plane k-3
+            if constexpr (ROLE == 0) {
+                const int zC = zA - 3;
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[j] = 0.f;
+                gs_octet<CK, H>(c_own + ring.s3, x_own + 2 * ST + prv, f_[1 - H], f_[H], f2, bz, acc, d);
+                if (k >= 6) {
+                    VT* ep = ek + ((long long)(sxy >> 1) * zC + ((g.nx >> 1) * gy + (gx >> 1)));
+                    if (in_a) st2<VT>(ep, make_float2(b_[1 - H][0], b_[1 - H][1]));
+                    if (in_b) st2<VT>(ep + 2, make_float2(b_[1 - H][2], b_[1 - H][3]));
+#pragma unroll
+                    for (int j = 0; j < 4; j++) pa[j] += acc[j];
+                }
+                if (k >= 5 && ((zC & 1) || zC + 1 == z1)) {
+                    // the pair's sums are complete (at k = 5 planes z0 and z0+1 become
+                    // the first pair)
+                    if (k >= 6) {
+                        if (gy & 1) put4(&S.ypart[(T.row - 3) >> 1][T.oc - 1].x, pa);
+                        copy4(ph, pa);
+                        rc_z = zC >> 1;
+                    }
+                    copy4(pa, pb);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) pb[j] = 0.f;
+                }
+                copy4(f_[H], f2);
+            }
+            copy4(b_[1 - H], b1);
+            if (ROLE == 0 || T.ring <= 1) put4(x_put + 2 * ST + cur, f2);
+        }
+        if (ROLE == 0 || T.ring < 4) put4(x_put + cur, r0);
+        if (ROLE == 0 || T.ring <= 2) put4(x_put + ST + cur, b1);
+        copy4(r_[H], r0);
+    };
+    // Straight-line steps in pairs of the two parities; a role's warps run the
+    // stages their octets take part in (0: all, 1: without the output stage,
+    // 2: the first two).  The first steps of a run work on planes that are not
+    // there yet: nothing valid reads their results.
+    auto run = [&](auto role) {
+        int k = 0;
+        if ((gy + zs) & 1) {
+            step(Phase<1>{}, role, 0);
+            block_bar();
+            k = 1;
+        }
+        for (;;) {
+            step(Phase<0>{}, role, k);
+            if (++k >= nsteps) break;
+            block_bar();
+            step(Phase<1>{}, role, k);
+            if (++k >= nsteps) break;
+            block_bar();
+        }
+    };
+    if (own_warp) run(Phase<0>{});
+    else run(Phase<1>{});
+    __syncthreads();
+    flush_rc();
+    ring.drain();
+    if (UPDATE) finish_residual_norm(rr_thread, sc, partials, nblocks, sh);
 }
 
-// ----------------------------------------------------- post-smoothing pass
-// See k_prolong_postsmooth; e, r and the coarse correction arrive through
-// tm_e, tm_r and tm_ec, the records through tm_rec.  Step structure as in
-// k_pre_tma.
+// ------------------------------------------------------------------ up pass
+// The black correction ek of the down pass plus w P ec, three half-steps, out
+// (VT).  DOT (finest level): r . out / sigma gives rz and beta; the next
+// V-cycle's sigma is then taken from ||r||^2.
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
-__global__ void __launch_bounds__(TGeo<CK>::NT, TMA_MIN_BLOCKS)
-    k_post_tma(const __grid_constant__ CUtensorMap tm_rec, const __grid_constant__ CUtensorMap tm_e,
-               const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_ec, Grid3 g,
-               VT* __restrict__ out, const VT* __restrict__ accum, float w, Scalars* sc, double* partials,
-               int nblocks, long long n_active) {
+__global__ void __launch_bounds__(OGeo<CK>::NT, 1)
+    k_post_tma(const __grid_constant__ CUtensorMap tm_rec, Grid3 g, Grid3 gc, const VT* __restrict__ ek,
+               const VTc* __restrict__ ec, const VT* __restrict__ rin, VT* __restrict__ out,
+               const VT* __restrict__ accum, float w, Scalars* sc, double* partials, int nblocks,
+               long long n_active) {
     if (sc->converged) return;
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    using SM = PostTmaSm<CK, VT, VTc>;
+    using ET = Entry;
+    using G = OGeo<CK>;
+    using SM = PassSm<CK>;
     using R4 = typename Raw4<VT>::T;
+    using P2 = typename Raw2<VT>::T;
     using C2 = typename Raw2<VTc>::T;
-    constexpr int FTY = G::FTY, NT = G::NT, RH = G::RH, NS = G::NS, SL = RH * RW;
-    constexpr unsigned BYTES = RH * RW * sizeof(CT) + 2 * RH * V::VW * sizeof(VT);
-    constexpr unsigned EC_BYTES = G::CRH * G::CW * sizeof(VTc);
+    constexpr int NT = G::NT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SM& S = aligned_smem<SM>(smem_raw);
     __shared__ double sh[NT / 32];
     const int t = threadIdx.x;
-    constexpr int ISSUER = NT - 1;
     const float sigma = FINE ? sc->sigma : 1.0f;
     const float is = FINE ? sc->inv_sigma : 1.0f;
-    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * FTY;
+    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * G::FTY;
     const int z0 = blockIdx.z * g.zper, z1 = min(g.nz, z0 + g.zper);
-    const int zs = z0 - 2, nsteps = z1 - z0 + 4;
-    const long long sxy = (long long)g.nx * g.ny;
-    int last_issued = 0;
-    auto issue = [&](int k, int off) {  // the copies of plane zs + k (and its coarse plane when it starts one)
-        const int zz = zs + k;
-        unsigned long long* b = &S.bar[k & 1];
-        fence_proxy_async();
-        mbar_expect_tx(b, BYTES + ((k & 1) ? 0u : EC_BYTES));
-        tma_4d(&S.c[0][0][0] + off, &tm_rec, 2 * x0 - 8, 0, y0 - 2, zz, b);
-        tma_3d(&S.ev[k & 1][0][0], &tm_e, x0 - V::XS, y0 - 2, zz, b);
-        tma_3d(&S.rv[k & 1][0][0], &tm_r, x0 - V::XS, y0 - 2, zz, b);
-        if (!(k & 1)) tma_3d(&S.ec[(k >> 1) & 1][0], &tm_ec, (x0 >> 1) - 8, (y0 >> 1) - 1, zz >> 1, b);
-        last_issued = k;
+    const int zs = z0 - 3, nsteps = z1 - z0 + 6;
+    const Octet<G> T(t);
+    const int gx = x0 - 8 + 8 * T.oc, gy = y0 - 3 + T.row;
+    const bool in_y = T.ring < 4 && gy >= 0 && gy < g.ny;
+    // of the side octets only the quad next to the tile is read
+    const bool in_a = in_y && T.oc != 0 && gx < g.nx, in_b = in_y && T.oc != NO - 1 && gx + 4 >= 0 && gx + 4 < g.nx;
+    const bool own_warp = octet_index(t) < G::C0;
+    const int sxy = g.nx * g.ny, go = gx + g.nx * gy;
+    const int ko = (gx >> 1) + (g.nx >> 1) * gy, co = (gx >> 1) + gc.nx * (gy >> 1), csxy = gc.nx * gc.ny;
+    const int rs = min(max(T.row, 1), G::RH - 2);
+    const ET* const c_own = &S.c[0][rs][4 * T.oc];
+    float* const x_own = &S.ex[0][0][rs][4 * T.oc];
+    float* const x_put = &S.ex[0][0][T.row][4 * T.oc];
+    constexpr int XP = G::RH * HH, ST = 2 * XP;
+    R4 rv[2];
+    P2 kv[2];
+    C2 cv[2];
+    auto load = [&](int zz) {  // right-hand side, black correction and coarse parents of plane zz
+        const bool okz = zz >= 0 && zz < g.nz;
+        const VT* rp = rin + ((long long)sxy * zz + go);
+        const VT* kp = ek + ((long long)(sxy >> 1) * zz + ko);
+        const VTc* cp = ec + ((long long)csxy * (zz >> 1) + co);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const bool ok = okz && (u ? in_b : in_a);
+            rv[u] = ldg_quad<VT>(rp + 4 * u, ok);
+            kv[u] = ldg_pair<VT>(kp + 2 * u, ok);
+            cv[u] = ldg_pair<VTc>(cp + 2 * u, ok);
+        }
     };
-    if (t == ISSUER) {
-        mbar_init(&S.bar[0], 1);
-        mbar_init(&S.bar[1], 1);
-        S.abort_ = 0;
-        fence_barrier_init();
-    }
-    __syncthreads();
-    if (t == ISSUER) issue(0, 0);
-
-    int r_row, r_q;
-    stage_task(t, RH, 0, &r_row, &r_q);
-    const bool has_red = t < G::NRED;
-    const int r_o = r_row * RW + 2 * r_q;
-    const int r_v = r_row * V::VW + V::VX + 4 * r_q;
-    const int r_c = (r_row >> 1) * G::CW + 6 + 2 * r_q;  // the quad's two coarse parents
-    const int r_gx = x0 - XO + 4 * r_q, r_gy = y0 - 2 + r_row;
-    const int r_par = r_gy & 1;
-    const bool r_inside = r_gx >= 0 && r_gx < g.nx && r_gy >= 0 && r_gy < g.ny;
-    int b_row, b_q;
-    stage_task(t, G::NBR, 1, &b_row, &b_q);
-    const bool has_blk = t < G::NBLK;
-    const int b_o = b_row * RW + 2 * b_q;
-    const int b_par = (y0 - 2 + b_row) & 1;
-    const bool has_own = t < G::NOWN;
-    const int tx = t % QX, ty = t / QX;
-    const int ox = x0 + 4 * tx, oy = y0 + ty;
-    const bool own_inside = has_own && ox < g.nx && oy < g.ny;
-    const int oo = (ty + 2) * RW + 2 * (tx + 1);
-    const int ov = (ty + 2) * V::VW + V::VX + 4 * (tx + 1);
-    const long long og = ox + (long long)g.nx * oy;
-    const CT* c0 = &S.c[0][0][0];
-    float* e0 = &S.ep[0][0][0];
-    Acc acc;
-    R4 rq_own[4];  // own quad's right-hand side of planes zA-3 .. zA (slot zA & 3)
-
-    int o0 = 0, o1 = (NS - 1) * SL, o2 = (NS - 2) * SL, o3 = (NS - 3) * SL;
-    auto step = [&](auto ph, int k) {
-        constexpr int P = decltype(ph)::value;
+    load(zs);
+    RecordRing<CK> ring(S, &tm_rec, x0, y0, zs);
+    Acc acc_rz;
+    // the octet's values by step parity: prolonged blacks (index 1-H: plane k-1,
+    // H: k-2), first reds (H: k-2, 1-H: k-3), changes of the blacks (1-H: k-3,
+    // H: k-4); right-hand sides: reds of plane k-1, blacks (1-H: k-1, H: k-2);
+    // smoothed blacks of plane k-3
+    float p_[2][4] = {}, r_[2][4] = {}, b_[2][4] = {}, gr1[4] = {}, gb_[2][4] = {}, zb[4] = {};
+    auto step = [&](auto hc, auto role, int k) {
+        constexpr int H = decltype(hc)::value;  // red half of plane k; the stages' cells sit at half 1 - H
+        constexpr int ROLE = decltype(role)::value;
         const int zA = zs + k;
-        const bool aborted = *reinterpret_cast<volatile int*>(&S.abort_) != 0;
-        if (t == ISSUER && k + 1 < nsteps && !aborted) issue(k + 1, o0 == (NS - 1) * SL ? 0 : o0 + SL);
-        if (!aborted && !mbar_wait(&S.bar[P & 1], P >> 1)) {
-            S.abort_ = 1;
-            sc->stalled = 1;
-            sc->converged = 1;
+        const int cur = (k & 1) * XP, prv = XP - cur;
+        ring.step(k, nsteps, sc);
+        // the right-hand side of plane k-3, for r . z
+        R4 rz[2];
+        const long long oC = (long long)sxy * (zA - 3) + go;
+        if (DOT && ROLE == 0) {
+            rz[0] = ldg_quad<VT>(rin + oC, k >= 6 && in_a);
+            rz[1] = ldg_quad<VT>(rin + oC + 4, k >= 6 && in_b);
         }
-        if (has_own) rq_own[P] = *reinterpret_cast<const R4*>(&S.rv[P & 1][0][0] + ov);
-        // ---- prolongation: plane zA over the 2-halo rows
-        if (has_red) {
-            float* EP = e0 + o0;
-            float4 ev = make_float4(0.f, 0.f, 0.f, 0.f), rq = ev;
-            float2 cv = make_float2(0.f, 0.f);
-            if (r_inside && zA >= 0 && zA < g.nz) {
-                ev = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.ev[P & 1][0][0] + r_v));
-                rq = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.rv[P & 1][0][0] + r_v));
-                cv = cvt2(*reinterpret_cast<const C2*>(&S.ec[P >> 1][0] + r_c));
-            }
-            const int p = r_par ^ (P & 1);
-            const float2 er = p ? make_float2(ev.y, ev.w) : make_float2(ev.x, ev.z);
-            const float2 rb = p ? make_float2(rq.x, rq.z) : make_float2(rq.y, rq.w);
-            *reinterpret_cast<float2*>(EP + r_o + p * HW) = make_float2(fmaf(w, cv.x, er.x), fmaf(w, cv.y, er.y));
-            *reinterpret_cast<float2*>(EP + r_o + (1 - p) * HW) = make_float2(sigma * rb.x, sigma * rb.y);
-        }
-        __syncthreads();
-        // ---- black half-step: plane zA-1 over the 1-halo rows, in place
-        if (has_blk && zA - 1 >= z0 - 1) {
-            const CT* C = c0 + o1;
-            const CT* CN = c0 + o0;
-            float* E = e0 + o1;
-            const float* EM = e0 + o2;
-            const float* EP = e0 + o0;
-            const int h = b_par ^ (P & 1);
-            const int o = b_o + h * HW;
-            float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, o, h, *reinterpret_cast<const float2*>(E + o), &d);
-            *reinterpret_cast<float2*>(E + o) = divide2(s, d);
-        }
-        __syncthreads();
-        // ---- red half-step: plane zA-2 over the tile, out = z
-        const int zC = zA - 2;
-        if (has_own && zC >= z0 && zC < z1) {
-            const CT* C = c0 + o2;
-            const CT* CN = c0 + o1;
-            const float* E = e0 + o2;
-            const float* EM = e0 + o3;
-            const float* EP = e0 + o1;
-            const int p = (oy & 1) ^ (P & 1);
-            const float4 rv = cvt4r<VT>(rq_own[(P + 2) & 3]);
-            const float2 rr = p ? make_float2(rv.y, rv.w) : make_float2(rv.x, rv.z);
-            float2 d;
-            const float2 s = gs_sum2<CK>(C, CN, E, EM, EP, oo + p * HW, p, make_float2(sigma * rr.x, sigma * rr.y), &d);
-            const float2 zr = divide2(s, d);
-            const float2 zb = *reinterpret_cast<const float2*>(E + oo + (1 - p) * HW);
-            float4 zv = p ? make_float4(zb.x, zr.x, zb.y, zr.y) : make_float4(zr.x, zb.x, zr.y, zb.y);
-            if (own_inside) {
-                if (accum) {  // out = accum + z (second W-cycle visit)
-                    const float4 a = cvt4r<VT>(*reinterpret_cast<const R4*>(accum + og + sxy * zC));
-                    zv = make_float4(a.x + zv.x, a.y + zv.y, a.z + zv.z, a.w + zv.w);
-                }
-                st4<VT>(out + og + sxy * zC, zv);
-                if (DOT) {
-                    acc.add_prod(rv.x, zv.x * is);
-                    acc.add_prod(rv.y, zv.y * is);
-                    acc.add_prod(rv.z, zv.z * is);
-                    acc.add_prod(rv.w, zv.w * is);
-                }
+        // ---- prolongation onto the black cells, plane k
+        float p0[4], gr0[4], gb0[4], bz[4];
+        {
+            const float4 ra = cvt4r<VT>(rv[0]), rb = cvt4r<VT>(rv[1]);
+            const float2 ka = cvt2(kv[0]), kb = cvt2(kv[1]), ca = cvt2(cv[0]), cb = cvt2(cv[1]);
+            load(zA + 1);
+            p0[0] = fmaf(w, ca.x, ka.x);
+            p0[1] = fmaf(w, ca.y, ka.y);
+            p0[2] = fmaf(w, cb.x, kb.x);
+            p0[3] = fmaf(w, cb.y, kb.y);
+            const float re[4] = {ra.x, ra.z, rb.x, rb.z}, rd[4] = {ra.y, ra.w, rb.y, rb.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                gr0[j] = sigma * (H ? rd[j] : re[j]);
+                gb0[j] = sigma * (H ? re[j] : rd[j]);
             }
         }
+        // ---- first red half-step, plane k-1
+        float r1[4], b2[4], acc[4], d[4];
+        rec_lo<CK>(ld_rec<CK>(c_own + ring.s0 + (3 - H) * HH), bz);  // z-high mobilities: plane k, the same half
+        copy4(acc, gr1);
+        gs_octet<CK, 1 - H>(c_own + ring.s1, x_own + prv, p_[1 - H], p_[H], p0, bz, acc, d);
+#pragma unroll
+        for (int j = 0; j < 4; j++) r1[j] = acc[j] * rcp_or_zero(d[j]);
+        copy4(gr1, gr0);
+        if constexpr (ROLE <= 1) {
+            // ---- black half-step, plane k-2: its change of the prolonged value
+            float zn[4];
+            copy4(acc, gb_[H]);
+            gs_octet<CK, 1 - H>(c_own + ring.s2, x_own + ST + prv, r_[H], r_[1 - H], r1, bz, acc, d);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float ri = rcp_or_zero(d[j]);
+                b2[j] = ri > 0.f ? SOR_BLACK * fmaf(acc[j], ri, -p_[H][j]) : -p_[H][j];
+                zn[j] = p_[H][j] + b2[j];
+            }
+            if constexpr (ROLE == 0) {
+                // ---- second red half-step, plane k-3, out = z: the red values move
+                // by the sum over the black changes
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[j] = 0.f;
+                gs_octet<CK, 1 - H>(c_own + ring.s3, x_own + 2 * ST + prv, b_[1 - H], b_[H], b2, bz, acc, d);
+                if (k >= 6) {
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const float za = fmaf(acc[2 * u], rcp_or_zero(d[2 * u]), r_[1 - H][2 * u]);
+                        const float zc = fmaf(acc[2 * u + 1], rcp_or_zero(d[2 * u + 1]), r_[1 - H][2 * u + 1]);
+                        // red cells at half 1 - H, black cells at half H
+                        float4 z4 = H ? make_float4(za, zb[2 * u], zc, zb[2 * u + 1])
+                                      : make_float4(zb[2 * u], za, zb[2 * u + 1], zc);
+                        if (!(u ? in_b : in_a)) continue;
+                        if (!DOT && accum) {  // out = accum + z (second W-cycle visit)
+                            const float4 a = cvt4r<VT>(*reinterpret_cast<const R4*>(accum + oC + 4 * u));
+                            z4 = make_float4(a.x + z4.x, a.y + z4.y, a.z + z4.z, a.w + z4.w);
+                        }
+                        st4<VT>(out + oC + 4 * u, z4);
+                        if (DOT) {
+                            const float4 r4 = cvt4r<VT>(rz[u]);
+                            acc_rz.add_prod(r4.x, z4.x * is);
+                            acc_rz.add_prod(r4.y, z4.y * is);
+                            acc_rz.add_prod(r4.z, z4.z * is);
+                            acc_rz.add_prod(r4.w, z4.w * is);
+                        }
+                    }
+                }
+                copy4(zb, zn);
+                copy4(b_[H], b2);
+            }
+            copy4(r_[1 - H], r1);
+            copy4(gb_[H], gb0);
+            if (ROLE == 0 || T.ring <= 1) put4(x_put + 2 * ST + cur, b2);
+        }
+        if (ROLE == 0 || T.ring < 4) put4(x_put + cur, p0);
+        if (ROLE == 0 || T.ring <= 2) put4(x_put + ST + cur, r1);
+        copy4(p_[H], p0);
     };
-    auto advance = [&]() {
-        o3 = o2;
-        o2 = o1;
-        o1 = o0;
-        o0 = o0 == (NS - 1) * SL ? 0 : o0 + SL;
+    // see k_pre_tma
+    auto run = [&](auto role) {
+        int k = 0;
+        if ((gy + zs) & 1) {
+            step(Phase<1>{}, role, 0);
+            block_bar();
+            k = 1;
+        }
+        for (;;) {
+            step(Phase<0>{}, role, k);
+            if (++k >= nsteps) break;
+            block_bar();
+            step(Phase<1>{}, role, k);
+            if (++k >= nsteps) break;
+            block_bar();
+        }
     };
-    for (int k = 0;;) {
-        step(Phase<0>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<1>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<2>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-        step(Phase<3>{}, k);
-        advance();
-        if (++k >= nsteps) break;
-    }
+    if (own_warp) run(Phase<0>{});
+    else run(Phase<1>{});
     __syncthreads();
-    if (t == ISSUER && S.abort_) (void)mbar_wait(&S.bar[last_issued & 1], (last_issued >> 1) & 1);
-    if (DOT) {
-        double v1[1] = {acc.total()};
-        block_sum<1>(v1, sh);
-        if (store_partials_is_last<1>(v1, partials, nblocks, &sc->ticket[9])) {
-            double tot[1];
-            finish_partials<1>(tot, partials, nblocks, sh, &sc->ticket[9]);
-            if (t == 0 && !sc->stalled) {
-                const double rz = tot[0];
-                if (!isfinite(rz)) {
-                    sc->nonfinite = 1;
-                    sc->converged = 1;
-                } else if (!(rz > 0.0)) {
-                    sc->breakdown = 1;
-                    sc->converged = 1;
-                } else if (sc->first) {
-                    sc->rz = rz;
-                    sc->beta = 0.0;
-                    sc->beta_f = 0.0f;
-                } else {
-                    sc->beta = rz / sc->rz;
-                    sc->beta_f = (float)sc->beta;
-                    sc->rz = rz;
-                }
-                sc->inv_sigma_z = sc->inv_sigma;
-                set_sigma_from(sc, sc->rr, n_active);
-            }
-        }
-    }
+    ring.drain();
+    if (DOT) finish_rz(acc_rz.total(), sc, partials, nblocks, n_active, sh);
 }
 
-// ------------------------------------------------- whole-run coarse passes
-// On a coarse level whose runs of two planes fill at most one wave of one
-// block per SM (the 64^3 and 32^3 levels below a 256^3 or 128^3 grid), a
-// z-marching pass is six plane steps of three dependent stages each, and the
-// stages' latency, not bandwidth, sets its time.  These kernels do the same
-// work with each stage over every plane of the run at once: the red (or
-// prolongation) stage over planes z0-2 .. z1+1, the black half-step over
-// z0-1 .. z1, the restriction (or last red half-step) over z0 .. z1-1, with a
-// barrier between stages.  Every plane's copies are issued when the block
-// starts, each plane on its own mbarrier.  The per-cell arithmetic and its
-// order are those of k_pre_tma / k_post_tma on coarse levels, so every
-// vector written is bit-identical.
+// ------------------------------------------------- records and residuals
+// Entries of a half row: nx/2, rounded up to 16 bytes.
+__host__ __device__ inline int rec_pitch(int nx) { return (nx / 2 + 3) / 4 * 4; }
+template <int CK>
+__device__ __forceinline__ float2 entry2(const Entry& e) {
+    return make_float2(half_lo<CK>(e), half_hi<CK>(e));
+}
+// (beta_x, beta_y) and (beta_z, diagonal) per cell from the level's
+// coefficient records (beta_x, beta_y, beta_z, reaction); the diagonal is the
+// FP32 sum of the record-precision values, rounded up to the record
+// precision (the operator stays diagonally dominant).  The betas are exact
+// in the record precision already.
+template <int CK>
+__global__ void __launch_bounds__(TILE_THREADS) k_tma_records(Grid3 g, const void* __restrict__ coef_v,
+                                                              void* __restrict__ sm_v) {
+    using CT = typename CoefStore<CK>::T;
+    using ET = Entry;
+    const CT* coef = reinterpret_cast<const CT*>(coef_v);
+    ET* sm = reinterpret_cast<ET*>(sm_v);
+    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    if (x >= g.nx || y >= g.ny) return;
+    const int z0 = blockIdx.z * g.zper, z1 = min(g.nz, z0 + g.zper);
+    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
+    const int pitch = rec_pitch(g.nx), h = x & 1;
+    for (int z = z0; z < z1; z++) {
+        const long long i = x + sy * y + sz * z;
+        const float4 c = unpack<CK>(coef[i]);
+        const float bxh = x + 1 < g.nx ? unpack<CK>(coef[i + 1]).x : 0.f;
+        const float byh = y + 1 < g.ny ? unpack<CK>(coef[i + sy]).y : 0.f;
+        const float bzh = z + 1 < g.nz ? unpack<CK>(coef[i + sz]).z : 0.f;
+        const float d = ((c.x + bxh) + (c.y + byh)) + ((c.z + bzh) + c.w);
+        ET* row = sm + (((long long)z * g.ny + y) * 4 + h) * pitch + (x >> 1);
+        const uint2 u = coef[i];
+        unsigned short dh;
+        if constexpr (CK == 1) {
+            const __half v = __float2half_ru(d);
+            dh = *reinterpret_cast<const unsigned short*>(&v);
+        } else {
+            const __nv_bfloat16 v = __float2bfloat16_ru(d);
+            dh = *reinterpret_cast<const unsigned short*>(&v);
+        }
+        row[0] = u.x;
+        row[2 * pitch] = (u.y & 0x0000ffffu) | ((unsigned)dh << 16);
+    }
+}
+// r2 = r - A e with the records' betas and diagonal: the right-hand side of a
+// W-cycle level's second visit.
 template <int CK, class VT>
-struct PreRunSm {
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    alignas(128) CT c[G::NP][G::RH][RW];
-    alignas(128) VT rv[G::NP][G::RH][V::VW];
-    alignas(16) float er[G::NP][G::RH][RW];
-    float2 ypart[G::FTY][QX];
-    unsigned long long bar[G::NP];
-    int abort_;
-};
-template <int CK, class VT, class VTc>
-struct PostRunSm {
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    static constexpr int ECS = padded128<VTc, G::CRH * G::CW>();
-    alignas(128) CT c[G::NP][G::RH][RW];
-    alignas(128) VT ev[G::NP][G::RH][V::VW];
-    alignas(128) VT rv[G::NP][G::RH][V::VW];
-    alignas(128) VTc ec[G::NP / 2][ECS];
-    alignas(16) float ep[G::NP][G::RH][RW];
-    unsigned long long bar[G::NP];
-    int abort_;
-};
-
-// Issue the copies of planes zs .. zs+np-1 (thread ISSUER) and wait for all of
-// them (every thread, bounded); false when a wait ran out.
-template <class SM, class IssueFn>
-__device__ __forceinline__ bool run_copies(SM& S, int np, int issuer, IssueFn issue_plane) {
-    const int t = threadIdx.x;
-    if (t == issuer) {
-        for (int k = 0; k < (int)(sizeof(S.bar) / sizeof(S.bar[0])); k++) mbar_init(&S.bar[k], 1);
-        S.abort_ = 0;
-        fence_barrier_init();
-    }
-    __syncthreads();
-    if (t == issuer)
-        for (int k = 0; k < np; k++) issue_plane(k, &S.bar[k]);
-    bool ok = true;
-    for (int k = 0; k < np && ok; k++) ok = mbar_wait(&S.bar[k], 0);
-    return ok;
-}
-// After a timed-out wait: the issuing thread waits (bounded) for every copy
-// it issued before the block exits.
-template <class SM>
-__device__ __forceinline__ void run_drain(SM& S, int np, int issuer) {
-    if (threadIdx.x == issuer && S.abort_)
-        for (int k = 0; k < np; k++) (void)mbar_wait(&S.bar[k], 0);
-}
-
-template <int CK, class VT, class VTc>
-__global__ void __launch_bounds__(TGeo<CK>::NT, 1)
-    k_pre_run(const __grid_constant__ CUtensorMap tm_rec, const __grid_constant__ CUtensorMap tm_r, Grid3 g,
-              Grid3 gc, VT* __restrict__ e, VTc* __restrict__ rc, Scalars* sc) {
+__global__ void __launch_bounds__(TILE_THREADS) k_tma_residual(Grid3 g, const void* __restrict__ sm_v,
+                                                               const VT* __restrict__ r, const VT* __restrict__ e,
+                                                               VT* __restrict__ r2, const Scalars* sc) {
     if (sc->converged) return;
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    using SM = PreRunSm<CK, VT>;
-    using R4 = typename Raw4<VT>::T;
-    constexpr int FTY = G::FTY, NT = G::NT, RH = G::RH, NP = G::NP, SL = RH * RW;
-    constexpr unsigned BYTES = RH * RW * sizeof(CT) + RH * V::VW * sizeof(VT);
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    SM& S = aligned_smem<SM>(smem_raw);
-    const int t = threadIdx.x;
-    constexpr int ISSUER = NT - 1;
-    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * FTY;
-    const int z0 = blockIdx.z * 2, z1 = min(g.nz, z0 + 2);
-    const int zs = z0 - 2, np = z1 - z0 + 4;  // planes zs .. z1+1; zs is even
-    const long long sxy = (long long)g.nx * g.ny;
-    const bool ok = run_copies(S, np, ISSUER, [&](int k, unsigned long long* b) {
-        fence_proxy_async();
-        mbar_expect_tx(b, BYTES);
-        tma_4d(&S.c[k][0][0], &tm_rec, 2 * x0 - 8, 0, y0 - 2, zs + k, b);
-        tma_3d(&S.rv[k][0][0], &tm_r, x0 - V::XS, y0 - 2, zs + k, b);
-    });
-    if (!ok) {
-        S.abort_ = 1;
-        sc->stalled = 1;
-        sc->converged = 1;
+    using ET = Entry;
+    const ET* sm = reinterpret_cast<const ET*>(sm_v);
+    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    if (x >= g.nx || y >= g.ny) return;
+    const int z0 = blockIdx.z * g.zper, z1 = min(g.nz, z0 + g.zper);
+    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
+    const int pitch = rec_pitch(g.nx), h = x & 1;
+    const long long rsy = 4ll * pitch, rsz = rsy * g.ny;
+    for (int z = z0; z < z1; z++) {
+        const long long i = x + sy * y + sz * z;
+        const ET* row = sm + rsz * z + rsy * y + (x >> 1);
+        const float2 a = entry2<CK>(row[h * pitch]), b = entry2<CK>(row[(2 + h) * pitch]);
+        const float bxh = x + 1 < g.nx ? entry2<CK>(row[(1 - h) * pitch + h]).x : 0.f;
+        const float byh = y + 1 < g.ny ? entry2<CK>(row[rsy + h * pitch]).y : 0.f;
+        const float bzh = z + 1 < g.nz ? entry2<CK>(row[rsz + (2 + h) * pitch]).x : 0.f;
+        float nsum = 0.f;
+        nsum = fmaf(a.x, x > 0 ? to_f(e[i - 1]) : 0.f, nsum);
+        nsum = fmaf(bxh, x + 1 < g.nx ? to_f(e[i + 1]) : 0.f, nsum);
+        nsum = fmaf(a.y, y > 0 ? to_f(e[i - sy]) : 0.f, nsum);
+        nsum = fmaf(byh, y + 1 < g.ny ? to_f(e[i + sy]) : 0.f, nsum);
+        nsum = fmaf(b.x, z > 0 ? to_f(e[i - sz]) : 0.f, nsum);
+        nsum = fmaf(bzh, z + 1 < g.nz ? to_f(e[i + sz]) : 0.f, nsum);
+        r2[i] = from_f<VT>(to_f(r[i]) - (b.y * to_f(e[i]) - nsum));
     }
-    const CT* c0 = &S.c[0][0][0];
-    float* e0 = &S.er[0][0][0];
-    // ---- red stage, planes 0 .. np-1 over the 2-halo rows
-    if (ok && t < G::NRED) {
-        int row, q;
-        stage_task(t, RH, 0, &row, &q);
-        const int o = row * RW + 2 * q, vo = row * V::VW + V::VX + 4 * q;
-        const int par = (y0 - 2 + row) & 1;
-#pragma unroll
-        for (int k = 0; k < NP; k++) {
-            if (k >= np) break;
-            const float4 rn = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.rv[k][0][0] + vo));
-            const int p = par ^ (k & 1);
-            float4 d0, d1;
-            rec2<CK>(c0 + k * SL + o + p * HW, &d0, &d1);
-            const float2 rr = p ? make_float2(rn.y, rn.w) : make_float2(rn.x, rn.z);
-            const float2 rb = p ? make_float2(rn.x, rn.z) : make_float2(rn.y, rn.w);
-            const float2 ev = divide2(make_float2(1.0f * rr.x, 1.0f * rr.y), make_float2(d0.w, d1.w));
-            *reinterpret_cast<float2*>(e0 + k * SL + o + p * HW) = ev;
-            *reinterpret_cast<float2*>(e0 + k * SL + o + (1 - p) * HW) = make_float2(1.0f * rb.x, 1.0f * rb.y);
-        }
-    }
-    __syncthreads();
-    // ---- black half-step, planes 1 .. np-2 over the 1-halo rows, in place
-    if (ok && t < G::NBLK) {
-        int row, q;
-        stage_task(t, G::NBR, 1, &row, &q);
-        const int ob = row * RW + 2 * q;
-        const int par = (y0 - 2 + row) & 1;
-#pragma unroll
-        for (int k = 1; k < NP - 1; k++) {
-            if (k > np - 2) break;
-            const int h = par ^ ((k + 1) & 1);
-            const int o = ob + h * HW;
-            float* E = e0 + k * SL;
-            float2 d;
-            const float2 s = gs_sum2<CK>(c0 + k * SL, c0 + (k + 1) * SL, E, E - SL, E + SL, o, h,
-                                         *reinterpret_cast<const float2*>(E + o), &d);
-            *reinterpret_cast<float2*>(E + o) = divide2(s, d);
-        }
-    }
-    __syncthreads();
-    // ---- correction out and restriction, planes 2 .. np-3 over the tile
-    const bool has_own = t < G::NOWN;
-    const int tx = t % QX, ty = t / QX;
-    const int ox = x0 + 4 * tx, oy = y0 + ty;
-    const bool own_inside = has_own && ox < g.nx && oy < g.ny;
-    const int oo = (ty + 2) * RW + 2 * (tx + 1);
-    const long long og = ox + (long long)g.nx * oy;
-    if (ok && has_own) {
-        float2 part = make_float2(0.f, 0.f);
-        for (int k = 2; k < np - 2; k++) {
-            const int zC = zs + k;
-            const float* E = e0 + k * SL;
-            const int p = (oy & 1) ^ (k & 1);
-            float2 d;
-            const float2 s = gs_sum2<CK>(c0 + k * SL, c0 + (k + 1) * SL, E, E - SL, E + SL, oo + p * HW, p,
-                                         make_float2(0.f, 0.f), &d);
-            part.x += s.x;
-            part.y += s.y;
-            if (own_inside) {
-                const float2 ev = *reinterpret_cast<const float2*>(E + oo);
-                const float2 od = *reinterpret_cast<const float2*>(E + oo + HW);
-                st4<VT>(e + (og + sxy * zC), make_float4(ev.x, od.x, ev.y, od.y));
-            }
-        }
-        S.ypart[ty][tx] = part;
-    }
-    __syncthreads();
-    if (ok && own_inside && !(ty & 1)) {
-        const float2 a = S.ypart[ty][tx], b = S.ypart[ty + 1][tx];
-        st2<VTc>(rc + (ox >> 1) + (long long)gc.nx * ((oy >> 1) + (long long)gc.ny * (z0 >> 1)),
-                 make_float2(0.25f * (a.x + b.x), 0.25f * (a.y + b.y)));
-    }
-    run_drain(S, np, ISSUER);
-}
-
-template <int CK, class VT, class VTc>
-__global__ void __launch_bounds__(TGeo<CK>::NT, 1)
-    k_post_run(const __grid_constant__ CUtensorMap tm_rec, const __grid_constant__ CUtensorMap tm_e,
-               const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_ec, Grid3 g,
-               VT* __restrict__ out, const VT* __restrict__ accum, float w, Scalars* sc) {
-    if (sc->converged) return;
-    using CT = typename CoefStore<CK>::T;
-    using G = TGeo<CK>;
-    using V = VGeo<VT>;
-    using SM = PostRunSm<CK, VT, VTc>;
-    using R4 = typename Raw4<VT>::T;
-    using C2 = typename Raw2<VTc>::T;
-    constexpr int FTY = G::FTY, NT = G::NT, RH = G::RH, NP = G::NP, SL = RH * RW;
-    constexpr unsigned BYTES = RH * RW * sizeof(CT) + 2 * RH * V::VW * sizeof(VT);
-    constexpr unsigned EC_BYTES = G::CRH * G::CW * sizeof(VTc);
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    SM& S = aligned_smem<SM>(smem_raw);
-    const int t = threadIdx.x;
-    constexpr int ISSUER = NT - 1;
-    const int x0 = blockIdx.x * PX, y0 = blockIdx.y * FTY;
-    const int z0 = blockIdx.z * 2, z1 = min(g.nz, z0 + 2);
-    const int zs = z0 - 2, np = z1 - z0 + 4;
-    const long long sxy = (long long)g.nx * g.ny;
-    const bool ok = run_copies(S, np, ISSUER, [&](int k, unsigned long long* b) {
-        const int zz = zs + k;
-        fence_proxy_async();
-        mbar_expect_tx(b, BYTES + ((k & 1) ? 0u : EC_BYTES));
-        tma_4d(&S.c[k][0][0], &tm_rec, 2 * x0 - 8, 0, y0 - 2, zz, b);
-        tma_3d(&S.ev[k][0][0], &tm_e, x0 - V::XS, y0 - 2, zz, b);
-        tma_3d(&S.rv[k][0][0], &tm_r, x0 - V::XS, y0 - 2, zz, b);
-        if (!(k & 1)) tma_3d(&S.ec[k >> 1][0], &tm_ec, (x0 >> 1) - 8, (y0 >> 1) - 1, zz >> 1, b);
-    });
-    if (!ok) {
-        S.abort_ = 1;
-        sc->stalled = 1;
-        sc->converged = 1;
-    }
-    const CT* c0 = &S.c[0][0][0];
-    float* e0 = &S.ep[0][0][0];
-    // ---- prolongation, planes 0 .. np-1 over the 2-halo rows
-    if (ok && t < G::NRED) {
-        int row, q;
-        stage_task(t, RH, 0, &row, &q);
-        const int o = row * RW + 2 * q, vo = row * V::VW + V::VX + 4 * q;
-        const int co = (row >> 1) * G::CW + 6 + 2 * q;  // the quad's two coarse parents
-        const int gx = x0 - XO + 4 * q, gy = y0 - 2 + row;
-        const int par = gy & 1;
-        const bool inside = gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny;
-#pragma unroll
-        for (int k = 0; k < NP; k++) {
-            if (k >= np) break;
-            const int zA = zs + k;
-            float4 ev = make_float4(0.f, 0.f, 0.f, 0.f), rq = ev;
-            float2 cv = make_float2(0.f, 0.f);
-            if (inside && zA >= 0 && zA < g.nz) {
-                ev = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.ev[k][0][0] + vo));
-                rq = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.rv[k][0][0] + vo));
-                cv = cvt2(*reinterpret_cast<const C2*>(&S.ec[k >> 1][0] + co));
-            }
-            const int p = par ^ (k & 1);
-            const float2 er = p ? make_float2(ev.y, ev.w) : make_float2(ev.x, ev.z);
-            const float2 rb = p ? make_float2(rq.x, rq.z) : make_float2(rq.y, rq.w);
-            float* EP = e0 + k * SL;
-            *reinterpret_cast<float2*>(EP + o + p * HW) = make_float2(fmaf(w, cv.x, er.x), fmaf(w, cv.y, er.y));
-            *reinterpret_cast<float2*>(EP + o + (1 - p) * HW) = make_float2(1.0f * rb.x, 1.0f * rb.y);
-        }
-    }
-    __syncthreads();
-    // ---- black half-step, planes 1 .. np-2 over the 1-halo rows, in place
-    if (ok && t < G::NBLK) {
-        int row, q;
-        stage_task(t, G::NBR, 1, &row, &q);
-        const int ob = row * RW + 2 * q;
-        const int par = (y0 - 2 + row) & 1;
-#pragma unroll
-        for (int k = 1; k < NP - 1; k++) {
-            if (k > np - 2) break;
-            const int h = par ^ ((k + 1) & 1);
-            const int o = ob + h * HW;
-            float* E = e0 + k * SL;
-            float2 d;
-            const float2 s = gs_sum2<CK>(c0 + k * SL, c0 + (k + 1) * SL, E, E - SL, E + SL, o, h,
-                                         *reinterpret_cast<const float2*>(E + o), &d);
-            *reinterpret_cast<float2*>(E + o) = divide2(s, d);
-        }
-    }
-    __syncthreads();
-    // ---- red half-step, planes 2 .. np-3 over the tile, out = z
-    if (ok && t < G::NOWN) {
-        const int tx = t % QX, ty = t / QX;
-        const int ox = x0 + 4 * tx, oy = y0 + ty;
-        const bool own_inside = ox < g.nx && oy < g.ny;
-        const int oo = (ty + 2) * RW + 2 * (tx + 1);
-        const int ov = (ty + 2) * V::VW + V::VX + 4 * (tx + 1);
-        const long long og = ox + (long long)g.nx * oy;
-        for (int k = 2; k < np - 2; k++) {
-            const int zC = zs + k;
-            const float* E = e0 + k * SL;
-            const int p = (oy & 1) ^ (k & 1);
-            const float4 rv = cvt4r<VT>(*reinterpret_cast<const R4*>(&S.rv[k][0][0] + ov));
-            const float2 rr = p ? make_float2(rv.y, rv.w) : make_float2(rv.x, rv.z);
-            float2 d;
-            const float2 s = gs_sum2<CK>(c0 + k * SL, c0 + (k + 1) * SL, E, E - SL, E + SL, oo + p * HW, p,
-                                         make_float2(1.0f * rr.x, 1.0f * rr.y), &d);
-            const float2 zr = divide2(s, d);
-            const float2 zb = *reinterpret_cast<const float2*>(E + oo + (1 - p) * HW);
-            float4 zv = p ? make_float4(zb.x, zr.x, zb.y, zr.y) : make_float4(zr.x, zb.x, zr.y, zb.y);
-            if (own_inside) {
-                if (accum) {  // out = accum + z (second W-cycle visit)
-                    const float4 a = cvt4r<VT>(*reinterpret_cast<const R4*>(accum + og + sxy * zC));
-                    zv = make_float4(a.x + zv.x, a.y + zv.y, a.z + zv.z, a.w + zv.w);
-                }
-                st4<VT>(out + og + sxy * zC, zv);
-            }
-        }
-    }
-    run_drain(S, np, ISSUER);
 }
 
 // ------------------------------------------------------------------ host
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 bool g_tma_enabled = false;
 int g_sms = 0;
-int g_occ[3][2][2] = {};  // [records precision][coarse level][pre / post]: resident blocks per SM
+int g_occ[3][2][2] = {};  // [records precision][coarse level][down / up]: resident blocks per SM
 
-bool encoder() {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-        else
-            (void)cudaGetLastError();
-    });
-    return g_encode != nullptr;
-}
-
-// 3-D map of a level vector (x-fastest cells, element size 4 or 2 bytes),
-// box w x rows x 1.
-bool vec_map(CUtensorMap* m, const void* base, int esize, const Grid3& g, int w, int rows) {
-    const cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.nx * esize, (cuuint64_t)g.nx * g.ny * esize};
-    const cuuint32_t box[3] = {(cuuint32_t)w, (cuuint32_t)rows, 1};
-    const cuuint32_t es[3] = {1, 1, 1};
-    return g_encode(m, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3,
-                    const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-// 4-D map of the split-row smoother records: (4 values x nx/2 records of a
-// half row, even/odd half, y, z), box 144 values x 2 halves x rows x 1.
+// 4-D map of the records: (entries of a half row, four half rows, y, z), box
+// HH x 4 x rows x 1; entries beyond nx/2 are out of bounds (zero).
 bool rec_map(CUtensorMap* m, const void* base, int ck, const Grid3& g, int rows) {
-    const int esize = ck == 0 ? 4 : 2;
-    const cuuint64_t half = (cuuint64_t)2 * g.nx;  // values per half row
-    const cuuint64_t dims[4] = {half, 2, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
-    const cuuint64_t strides[3] = {half * esize, 2 * half * esize, 2 * half * esize * g.ny};
-    const cuuint32_t box[4] = {(cuuint32_t)(2 * RW), 2, (cuuint32_t)rows, 1};
-    const cuuint32_t es[4] = {1, 1, 1, 1};
-    return g_encode(m, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 4,
-                    const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t es = 4;
+    const cuuint64_t half = (cuuint64_t)rec_pitch(g.nx) * es;
+    const cuuint64_t dims[4] = {(cuuint64_t)(g.nx / 2), 4, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
+    const cuuint64_t strides[3] = {half, 4 * half, 4 * half * g.ny};
+    const cuuint32_t box[4] = {(cuuint32_t)HH, 4, (cuuint32_t)rows, 1};
+    const cuuint32_t unit[4] = {1, 1, 1, 1};
+    return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4,
+                    const_cast<void*>(base), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// z runs as in fused_launch: even runs that fill whole waves of resident
-// blocks, each run computing two planes below and above it.
+// Even z runs that fill whole waves of resident blocks; each run computes
+// three planes below and above it.
 Launch tma_launch(const Grid3& g0, int fty, int nt, int occ) {
     Launch P;
     P.g = g0;
@@ -958,7 +792,7 @@ Launch tma_launch(const Grid3& g0, int fty, int nt, int occ) {
         const long long blocks = (long long)tiles * zcr;
         if (blocks > MAX_REDUCE_BLOCKS) break;
         const double waves = (double)blocks / cap;
-        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 4));
+        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 6));
         if (score > best) {
             best = score;
             best_zper = zper;
@@ -972,74 +806,25 @@ Launch tma_launch(const Grid3& g0, int fty, int nt, int occ) {
 }
 
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-bool pre_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q, float* r_out, void* e,
+void pre_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q, float* r_out, void* e,
              void* rc, Scalars* sc, double* partials, cudaStream_t s) {
-    using G = TGeo<CK>;
-    if (!aligned16(sm) || !aligned16(rin) || (UPDATE && !aligned16(q))) return false;
-    CUtensorMap tm_rec, tm_r, tm_q;
-    if (!rec_map(&tm_rec, sm, CK, g, G::RH)) return false;
-    if (!vec_map(&tm_r, rin, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    if (UPDATE) {
-        if (!vec_map(&tm_q, q, 4, g, VGeo<float>::VW, G::RH)) return false;
-    } else {
-        tm_q = tm_r;
-    }
+    using G = OGeo<CK>;
+    CUtensorMap tm_rec;
+    (void)rec_map(&tm_rec, sm, CK, g, G::RH);  // the same encode succeeded at tma_level_init
     const Launch P = tma_launch(g, G::FTY, G::NT, g_occ[CK][FINE ? 0 : 1][0]);
-    k_pre_tma<CK, VT, VTc, UPDATE, FINE><<<P.grid, P.block, sizeof(PreTmaSm<CK, VT, UPDATE>) + 128, s>>>(
-        tm_rec, tm_r, tm_q, P.g, gc, r_out, (VT*)e, (VTc*)rc, sc, partials, P.nblocks);
-    return true;
+    k_pre_tma<CK, VT, VTc, UPDATE, FINE><<<P.grid, P.block, sizeof(PassSm<CK>) + 128, s>>>(
+        tm_rec, P.g, gc, (const VT*)rin, q, r_out, (VT*)e, (VTc*)rc, sc, partials, P.nblocks);
 }
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
-bool post_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r, void* out,
+void post_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r, void* out,
               const void* accum, float w, Scalars* sc, double* partials, long long n_active, cudaStream_t s) {
-    using G = TGeo<CK>;
-    if (!aligned16(sm) || !aligned16(e) || !aligned16(r) || !aligned16(ec)) return false;
-    if ((gc.nx * (int)sizeof(VTc)) % 16) return false;
-    CUtensorMap tm_rec, tm_e, tm_r, tm_ec;
-    if (!rec_map(&tm_rec, sm, CK, g, G::RH)) return false;
-    if (!vec_map(&tm_e, e, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    if (!vec_map(&tm_r, r, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    if (!vec_map(&tm_ec, ec, (int)sizeof(VTc), gc, G::CW, G::CRH)) return false;
+    using G = OGeo<CK>;
+    CUtensorMap tm_rec;
+    (void)rec_map(&tm_rec, sm, CK, g, G::RH);  // the same encode succeeded at tma_level_init
     const Launch P = tma_launch(g, G::FTY, G::NT, g_occ[CK][FINE ? 0 : 1][1]);
-    k_post_tma<CK, VT, VTc, DOT, FINE><<<P.grid, P.block, sizeof(PostTmaSm<CK, VT, VTc>) + 128, s>>>(
-        tm_rec, tm_e, tm_r, tm_ec, P.g, (VT*)out, (const VT*)accum, w, sc, partials, P.nblocks, n_active);
-    return true;
-}
-
-// Coarse levels whose runs of two planes fill at most one wave of one block
-// per SM take the whole-run passes.
-bool whole_runs(const Grid3& g, int fty) {
-    const long long tiles = (long long)((g.nx + PX - 1) / PX) * ((g.ny + fty - 1) / fty);
-    return tiles * ((g.nz + 1) / 2) <= (g_sms > 0 ? g_sms : 152);
-}
-template <int CK, class VT, class VTc>
-bool pre_run(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, void* e, void* rc, Scalars* sc,
-             cudaStream_t s) {
-    using G = TGeo<CK>;
-    if (!aligned16(sm) || !aligned16(rin)) return false;
-    CUtensorMap tm_rec, tm_r;
-    if (!rec_map(&tm_rec, sm, CK, g, G::RH)) return false;
-    if (!vec_map(&tm_r, rin, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    const dim3 grid((g.nx + PX - 1) / PX, (g.ny + G::FTY - 1) / G::FTY, (g.nz + 1) / 2);
-    k_pre_run<CK, VT, VTc><<<grid, G::NT, sizeof(PreRunSm<CK, VT>) + 128, s>>>(tm_rec, tm_r, g, gc, (VT*)e,
-                                                                              (VTc*)rc, sc);
-    return true;
-}
-template <int CK, class VT, class VTc>
-bool post_run(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r, void* out,
-              const void* accum, float w, Scalars* sc, cudaStream_t s) {
-    using G = TGeo<CK>;
-    if (!aligned16(sm) || !aligned16(e) || !aligned16(r) || !aligned16(ec)) return false;
-    if ((gc.nx * (int)sizeof(VTc)) % 16) return false;
-    CUtensorMap tm_rec, tm_e, tm_r, tm_ec;
-    if (!rec_map(&tm_rec, sm, CK, g, G::RH)) return false;
-    if (!vec_map(&tm_e, e, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    if (!vec_map(&tm_r, r, (int)sizeof(VT), g, VGeo<VT>::VW, G::RH)) return false;
-    if (!vec_map(&tm_ec, ec, (int)sizeof(VTc), gc, G::CW, G::CRH)) return false;
-    const dim3 grid((g.nx + PX - 1) / PX, (g.ny + G::FTY - 1) / G::FTY, (g.nz + 1) / 2);
-    k_post_run<CK, VT, VTc><<<grid, G::NT, sizeof(PostRunSm<CK, VT, VTc>) + 128, s>>>(
-        tm_rec, tm_e, tm_r, tm_ec, g, (VT*)out, (const VT*)accum, w, sc);
-    return true;
+    k_post_tma<CK, VT, VTc, DOT, FINE><<<P.grid, P.block, sizeof(PassSm<CK>) + 128, s>>>(
+        tm_rec, P.g, gc, (const VT*)e, (const VTc*)ec, (const VT*)r, (VT*)out, (const VT*)accum, w, sc, partials,
+        P.nblocks, n_active);
 }
 
 template <class F>
@@ -1050,97 +835,96 @@ cudaError_t prep(F* fn, size_t bytes, int threads, int* occ) {
 }
 template <int CK, class VT, class VTc>
 cudaError_t prep_level(bool fine) {
-    using G = TGeo<CK>;
+    using G = OGeo<CK>;
     cudaError_t e = cudaSuccess;
-    const size_t pre_u = sizeof(PreTmaSm<CK, VT, true>) + 128, pre_n = sizeof(PreTmaSm<CK, VT, false>) + 128;
-    const size_t post = sizeof(PostTmaSm<CK, VT, VTc>) + 128;
+    const size_t bytes = sizeof(PassSm<CK>) + 128;
     if (fine) {
-        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, true, true>, pre_u, G::NT, &g_occ[CK][0][0]);
-        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, false, true>, pre_n, G::NT, nullptr);
-        if (e == cudaSuccess) e = prep(k_post_tma<CK, VT, VTc, true, true>, post, G::NT, &g_occ[CK][0][1]);
+        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, true, true>, bytes, G::NT, &g_occ[CK][0][0]);
+        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, false, true>, bytes, G::NT, nullptr);
+        if (e == cudaSuccess) e = prep(k_post_tma<CK, VT, VTc, true, true>, bytes, G::NT, &g_occ[CK][0][1]);
     } else {
-        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, false, false>, pre_n, G::NT, &g_occ[CK][1][0]);
-        if (e == cudaSuccess) e = prep(k_post_tma<CK, VT, VTc, false, false>, post, G::NT, &g_occ[CK][1][1]);
-        if (e == cudaSuccess) e = prep(k_pre_run<CK, VT, VTc>, sizeof(PreRunSm<CK, VT>) + 128, G::NT, nullptr);
-        if (e == cudaSuccess)
-            e = prep(k_post_run<CK, VT, VTc>, sizeof(PostRunSm<CK, VT, VTc>) + 128, G::NT, nullptr);
+        if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, false, false>, bytes, G::NT, &g_occ[CK][1][0]);
+        if (e == cudaSuccess) e = prep(k_post_tma<CK, VT, VTc, false, false>, bytes, G::NT, &g_occ[CK][1][1]);
     }
     return e;
 }
 }  // namespace
 
-bool tma_fused_enabled() { return g_tma_enabled; }
+PFN_cuTensorMapEncodeTiled_v12000 tma::encoder() {
+    static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+        (void)cudaGetLastError();
+        return static_cast<PFN_cuTensorMapEncodeTiled_v12000>(nullptr);
+    }();
+    return fn;
+}
 
 cudaError_t tma_prepare_attributes() {
     const char* ev = getenv("MHDPROJ_TMA");
-    g_tma_enabled = !(ev && ev[0] == '0') && encoder();
+    g_tma_enabled = !(ev && ev[0] == '0') && encoder() != nullptr;
     if (!g_tma_enabled) return cudaSuccess;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = prep_level<0, float, float>(true);
     if (e == cudaSuccess) e = prep_level<1, float, __half>(true);
     if (e == cudaSuccess) e = prep_level<2, float, __nv_bfloat16>(true);
-    if (e == cudaSuccess) e = prep_level<0, float, float>(false);
     if (e == cudaSuccess) e = prep_level<1, __half, __half>(false);
     if (e == cudaSuccess) e = prep_level<2, __nv_bfloat16, __nv_bfloat16>(false);
     return e;
 }
 
-static bool tma_grid_ok(const Grid3& g, int vt_bytes) {
-    return g_tma_enabled && g.periodic == 0 && g.nx % 4 == 0 && (g.nx * vt_bytes) % 16 == 0;
+bool tma_level_ok(const Grid3& g) { return g_tma_enabled && g.periodic == 0 && g.nx % 4 == 0; }
+bool tma_level_init(int ck, const Grid3& g, const void* sm) {
+    CUtensorMap tm;
+    return tma_level_ok(g) && rec_map(&tm, sm, ck, g, OGeo<1>::RH);
+}
+size_t tma_record_bytes(const Grid3& g) { return (size_t)g.ny * g.nz * 4 * rec_pitch(g.nx) * sizeof(Entry); }
+void tma_records(int ck, const Launch& L, const void* coef, void* sm, cudaStream_t s) {
+    if (ck == 1) k_tma_records<1><<<L.grid, L.block, 0, s>>>(L.g, coef, sm);
+    else k_tma_records<2><<<L.grid, L.block, 0, s>>>(L.g, coef, sm);
+}
+void tma_level_residual(int ck, const Launch& L, const void* sm, const void* r, const void* e, void* r2,
+                        const Scalars* sc, cudaStream_t s) {
+    if (ck == 1)
+        k_tma_residual<1, __half><<<L.grid, L.block, 0, s>>>(L.g, sm, (const __half*)r, (const __half*)e, (__half*)r2, sc);
+    else
+        k_tma_residual<2, __nv_bfloat16><<<L.grid, L.block, 0, s>>>(L.g, sm, (const __nv_bfloat16*)r,
+                                                                    (const __nv_bfloat16*)e, (__nv_bfloat16*)r2, sc);
 }
 
-bool tma_pre(int ck, bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin,
+#define MHDPROJ_TMA_PRE(CK, VT, VTc, UPD, FINE) \
+    pre_tma<CK, VT, VTc, UPD, FINE>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s)
+void tma_pre(int ck, bool fine, bool update, const Grid3& g, const Grid3& gc, const void* sm, const void* rin,
              const float* q, float* r_out, void* e, void* rc, Scalars* sc, double* partials, cudaStream_t s) {
-    const int vt = fine || ck == 0 ? 4 : 2;
-    if (!tma_grid_ok(g, vt)) return false;
-    if (fine) {
-        if (ck == 1)
-            return update ? pre_tma<1, float, __half, true, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s)
-                          : pre_tma<1, float, __half, false, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
-        if (ck == 2)
-            return update
-                       ? pre_tma<2, float, __nv_bfloat16, true, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s)
-                       : pre_tma<2, float, __nv_bfloat16, false, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
-        return update ? pre_tma<0, float, float, true, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s)
-                      : pre_tma<0, float, float, false, true>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
+    if (fine && update) {
+        if (ck == 1) MHDPROJ_TMA_PRE(1, float, __half, true, true);
+        else MHDPROJ_TMA_PRE(2, float, __nv_bfloat16, true, true);
+    } else if (fine) {
+        if (ck == 1) MHDPROJ_TMA_PRE(1, float, __half, false, true);
+        else MHDPROJ_TMA_PRE(2, float, __nv_bfloat16, false, true);
+    } else {
+        if (ck == 1) MHDPROJ_TMA_PRE(1, __half, __half, false, false);
+        else MHDPROJ_TMA_PRE(2, __nv_bfloat16, __nv_bfloat16, false, false);
     }
-    if (whole_runs(g, ck == 0 ? TGeo<0>::FTY : TGeo<1>::FTY)) {
-        if (ck == 1) return pre_run<1, __half, __half>(g, gc, sm, rin, e, rc, sc, s);
-        if (ck == 2) return pre_run<2, __nv_bfloat16, __nv_bfloat16>(g, gc, sm, rin, e, rc, sc, s);
-        return pre_run<0, float, float>(g, gc, sm, rin, e, rc, sc, s);
-    }
-    if (ck == 1) return pre_tma<1, __half, __half, false, false>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
-    if (ck == 2)
-        return pre_tma<2, __nv_bfloat16, __nv_bfloat16, false, false>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
-    return pre_tma<0, float, float, false, false>(g, gc, sm, rin, q, r_out, e, rc, sc, partials, s);
 }
-
-bool tma_post(int ck, bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
+#undef MHDPROJ_TMA_PRE
+#define MHDPROJ_TMA_POST(CK, VT, VTc, DOT, FINE) \
+    post_tma<CK, VT, VTc, DOT, FINE>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s)
+void tma_post(int ck, bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
               const void* r, void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active,
               cudaStream_t s) {
-    const int vt = fine || ck == 0 ? 4 : 2;
-    if (!tma_grid_ok(g, vt)) return false;
     if (fine) {
-        if (ck == 1)
-            return post_tma<1, float, __half, true, true>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
-        if (ck == 2)
-            return post_tma<2, float, __nv_bfloat16, true, true>(g, gc, sm, e, ec, r, out, accum, w, sc, partials,
-                                                                 n_active, s);
-        return post_tma<0, float, float, true, true>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
+        if (ck == 1) MHDPROJ_TMA_POST(1, float, __half, true, true);
+        else MHDPROJ_TMA_POST(2, float, __nv_bfloat16, true, true);
+    } else {
+        if (ck == 1) MHDPROJ_TMA_POST(1, __half, __half, false, false);
+        else MHDPROJ_TMA_POST(2, __nv_bfloat16, __nv_bfloat16, false, false);
     }
-    if (whole_runs(g, ck == 0 ? TGeo<0>::FTY : TGeo<1>::FTY)) {
-        if (ck == 1) return post_run<1, __half, __half>(g, gc, sm, e, ec, r, out, accum, w, sc, s);
-        if (ck == 2) return post_run<2, __nv_bfloat16, __nv_bfloat16>(g, gc, sm, e, ec, r, out, accum, w, sc, s);
-        return post_run<0, float, float>(g, gc, sm, e, ec, r, out, accum, w, sc, s);
-    }
-    if (ck == 1)
-        return post_tma<1, __half, __half, false, false>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
-    if (ck == 2)
-        return post_tma<2, __nv_bfloat16, __nv_bfloat16, false, false>(g, gc, sm, e, ec, r, out, accum, w, sc,
-                                                                       partials, n_active, s);
-    return post_tma<0, float, float, false, false>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
 }
+#undef MHDPROJ_TMA_POST
 
 }  // namespace mhdproj
