@@ -295,33 +295,33 @@ __device__ __forceinline__ float4 cmix4(float4 a, float4 b) {
 }
 
 // 256-lane tree in the shader's pairing (lane l absorbs lane l+s for
-// s = 128, 64, ..., 1); the last five levels are warp shuffles with the same
-// pairing.  The result is valid in thread 0.
-template <int OP>
-__device__ __forceinline__ float4 tree256(float4 v) {
-    __shared__ float4 red[kBlock];
+// s = 128, 64, ..., 1): one barrier, then a lane of the first warp forms the
+// first three levels from its eight leaves and the last five are warp
+// shuffles.  The result is valid in thread 0.  A second tree in a kernel needs
+// a barrier before it.
+__device__ __forceinline__ float comb(int, float a, float b) { return a + b; }
+__device__ __forceinline__ float2 comb(int, float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float4 comb(int op, float4 a, float4 b) { return op == 0 ? add4(a, b) : coef4(a, b); }
+__device__ __forceinline__ float down(float v, int s) { return __shfl_down_sync(0xffffffffu, v, s); }
+__device__ __forceinline__ float2 down(float2 v, int s) { return make_float2(down(v.x, s), down(v.y, s)); }
+__device__ __forceinline__ float4 down(float4 v, int s) {
+    return make_float4(down(v.x, s), down(v.y, s), down(v.z, s), down(v.w, s));
+}
+template <int OP, class T>
+__device__ __forceinline__ T tree256(T v) {
+    __shared__ T red[kBlock];
     const int l = threadIdx.x;
     red[l] = v;
     __syncthreads();
-#pragma unroll
-    for (int s = kBlock / 2; s >= 32; s >>= 1) {
-        if (l < s) red[l] = OP == 0 ? add4(red[l], red[l + s]) : coef4(red[l], red[l + s]);
-        __syncthreads();
-    }
-    float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (l < 32) {
-        w = red[l];
+        T a[4];
 #pragma unroll
-        for (int s = 16; s > 0; s >>= 1) {
-            float4 o;
-            o.x = __shfl_down_sync(0xffffffffu, w.x, s);
-            o.y = __shfl_down_sync(0xffffffffu, w.y, s);
-            o.z = __shfl_down_sync(0xffffffffu, w.z, s);
-            o.w = __shfl_down_sync(0xffffffffu, w.w, s);
-            w = OP == 0 ? add4(w, o) : coef4(w, o);
-        }
+        for (int k = 0; k < 4; k++) a[k] = comb(OP, red[l + 32 * k], red[l + 32 * k + 128]);
+        v = comb(OP, comb(OP, a[0], a[2]), comb(OP, a[1], a[3]));
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) v = comb(OP, v, down(v, s));
     }
-    return w;
+    return v;
 }
 // Single-block reduce over n partials: lane l accumulates l, l+256, ... from
 // `init` in that order (loads issued eight at a time), then the tree.
@@ -547,77 +547,164 @@ __global__ void __launch_bounds__(kBlock) k_em_initial_reduce(EmDev D) {
     D.scalars[0] = make_float4(sum.x, sum.y, sum.z, threshold);
     D.scalars[1] = make_float4(next != scale ? next : 0.0f, 0.0f, 0.0f, sum.y <= threshold ? 1.0f : 0.0f);
 }
+// ------------------------------------------------------------ CG iteration
+// The operator is bound by issue and by the latency of its sums (one edge a
+// thread: with four, or in blocks of 1024, the threads at conductors hold up
+// the others, 65 and 77 us), the residual and search passes by L2 and HBM
+// traffic (nine and four floats an edge; the 96^3 problem's arrays just exceed
+// what L2 keeps), for which a thread takes kEdges edges 256 apart so that their
+// loads are in flight together.  The sums of a group are scalars or pairs in the
+// shader's order.  96^3, microseconds an iteration, before and now: operator
+// 36 32, alpha 9.3 6.0, residual 26.5 21.7, beta 9.3 6.1, search 15 8.4.  The
+// reductions inside the passes, by the block that arrives last, cost more than
+// their launches (operator 44, residual 31).
+constexpr int kEdges = 4;
+// From here on kEdges edges a thread, one below: two blocks per SM of the long
+// form (28x28x23, 61 thousand edges, 57 blocks of it: 998 us a step against 926).
+constexpr uint32_t kManyEdges = 2u * 152u * kEdges * kBlock;
+// final_reduce over one or two sums per group, the same order.
+__device__ __forceinline__ void clear(float& v) { v = 0.0f; }
+__device__ __forceinline__ void clear(float2& v) { v = make_float2(0.0f, 0.0f); }
+template <class T>
+__device__ __forceinline__ T sum_reduce(const T* partials, uint32_t n) {
+    constexpr int U = 16;
+    T v;
+    clear(v);
+    uint32_t i = threadIdx.x;
+    for (; i + (U - 1) * kBlock < n; i += U * kBlock) {
+        T t[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) t[k] = __ldcg(partials + i + k * kBlock);
+#pragma unroll
+        for (int k = 0; k < U; k++) v = comb(0, v, t[k]);
+    }
+    for (; i < n; i += kBlock) v = comb(0, v, __ldcg(partials + i));
+    return tree256<0>(v);
+}
+
 // apply_operator (induction.wgsl:168-190); AIR = 0 forces the full operator.
+// An air edge's six neighbours exist.
 template <bool AIR>
 __global__ void __launch_bounds__(kBlock) k_em_apply(EmDev D) {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     float dot = 0.0f;
     if (i < D.E && active(D)) {
+        const float* __restrict__ p = D.p;
+        const float c = p[i];
         float q;
         if (AIR && (D.flags[i] & 4)) {
-            int axis = 0;
-            if (i >= D.e[0]) {
-                axis = 1;
-                if (i >= D.e[0] + D.e[1]) axis = 2;
-            }
-            uint32_t d[3];
-            edge_dims(D, axis, d);
-            const uint32_t zs = d[0] * d[1];
-            const float c = D.p[i];
+            const int axis = (i >= D.e[0]) + (i >= D.e[0] + D.e[1]);
+            const uint32_t ys = D.n[0] + (axis != 0), zs = ys * (D.n[1] + (axis != 1));
             float result = 0.0f;
-            result += (c - D.p[i - 1]) + (c - D.p[i + 1]);
-            result += (c - D.p[i - d[0]]) + (c - D.p[i + d[0]]);
-            result += (c - D.p[i - zs]) + (c - D.p[i + zs]);
+            result += (c - p[i - 1]) + (c - p[i + 1]);
+            result += (c - p[i - ys]) + (c - p[i + ys]);
+            result += (c - p[i - zs]) + (c - p[i + zs]);
             q = result;
         } else {
             q = EM_BY_AXIS(apply_edge, D, i);
         }
         D.w[i] = q;
-        dot = D.p[i] * q;
+        dot = c * q;
     }
-    const float4 t = tree256<0>(make_float4(dot, 0.0f, 0.0f, 0.0f));
-    if (threadIdx.x == 0) D.partials[blockIdx.x] = t;
+    const float t = tree256<0>(dot);
+    float* part = reinterpret_cast<float*>(D.partials);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 __global__ void __launch_bounds__(kBlock) k_em_alpha_reduce(EmDev D) {
-    const float4 sum = final_reduce<0>(D.partials, groups_of(D.E), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+    const float sum = sum_reduce(reinterpret_cast<const float*>(D.partials), groups_of(D.E));
     if (threadIdx.x == 0 && D.scalars[1].w == 0.0f) {
-        if (sum.x <= 0.0f || fabsf(sum.x) > 3e38f) D.scalars[1].w = 2.0f;
-        else D.scalars[1].x = D.scalars[0].x / sum.x;
+        if (sum <= 0.0f || fabsf(sum) > 3e38f) D.scalars[1].w = 2.0f;
+        else D.scalars[1].x = D.scalars[0].x / sum;
     }
 }
-// update_residual (induction.wgsl:197-208)
+__device__ __forceinline__ void set_beta(const EmDev& D, float2 sum) {
+    if (D.scalars[1].w != 0.0f) return;
+    D.scalars[1].y = sum.x / D.scalars[0].x;
+    D.scalars[0].x = sum.x;
+    D.scalars[0].y = sum.y;
+    D.scalars[1].z += 1.0f;
+    if (sum.y <= D.scalars[0].w) D.scalars[1].w = 1.0f;
+    if (fabsf(sum.x) > 3e38f || fabsf(sum.y) > 3e38f) D.scalars[1].w = 2.0f;
+}
+// update_residual (induction.wgsl:197-208); with the nodal correction that pass
+// sums instead (k_em_nodal, k_em_beta_reduce).
+template <int N, bool SUM>
 __global__ void __launch_bounds__(kBlock) k_em_update_residual(EmDev D) {
-    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < D.E && active(D)) {
-        const float alpha = D.scalars[1].x;
-        const float r = D.r[i] - alpha * D.w[i];
-        const float d = diagonal(D, i);
-        D.x[i] = D.x[i] + residual_scale(D) * (alpha * D.p[i]);
-        D.r[i] = r;
-        D.w[i] = d;
-        v = make_float4(r * r / d, r * r, 0.0f, 0.0f);
+    const uint32_t base = blockIdx.x * (N * kBlock) + threadIdx.x;
+    float rz[N] = {}, rr[N] = {};
+    if (active(D)) {
+        const float alpha = D.scalars[1].x, scale = residual_scale(D);
+        float r[N], w[N], d[N], x[N], pv[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const uint32_t i = base + k * kBlock;
+            if (i >= D.E) continue;
+            r[k] = D.r[i];
+            w[k] = D.w[i];
+            d[k] = diagonal(D, i);
+            x[k] = D.x[i];
+            pv[k] = D.p[i];
+        }
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const uint32_t i = base + k * kBlock;
+            if (i < D.E) {
+                const float rn = r[k] - alpha * w[k];
+                D.x[i] = x[k] + scale * (alpha * pv[k]);
+                D.r[i] = rn;
+                D.w[i] = d[k];
+                rz[k] = rn * rn / d[k];
+                rr[k] = rn * rn;
+            }
+        }
     }
-    const float4 t = tree256<0>(v);
-    if (threadIdx.x == 0) D.partials[blockIdx.x] = t;
+    if (!SUM) return;
+    float2* part = reinterpret_cast<float2*>(D.partials);
+    const uint32_t ng = groups_of(D.E);
+    if constexpr (N == 1) {
+        const float2 s = tree256<0>(make_float2(rz[0], rr[0]));
+        if (threadIdx.x == 0) part[blockIdx.x] = s;
+    } else {
+        static_assert(N == 4, "two pairs a tree");
+        const float4 a = tree256<0>(make_float4(rz[0], rr[0], rz[1], rr[1]));
+        __syncthreads();
+        const float4 b = tree256<0>(make_float4(rz[2], rr[2], rz[3], rr[3]));
+        if (threadIdx.x == 0) {
+            const float2 s[N] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y),
+                                 make_float2(b.z, b.w)};
+#pragma unroll
+            for (int k = 0; k < N; k++)
+                if (blockIdx.x * N + k < ng) part[blockIdx.x * N + k] = s[k];
+        }
+    }
+}
+__global__ void __launch_bounds__(kBlock) k_em_beta_reduce_pairs(EmDev D) {
+    const float2 sum = sum_reduce(reinterpret_cast<const float2*>(D.partials), groups_of(D.E));
+    if (threadIdx.x == 0) set_beta(D, sum);
 }
 __global__ void __launch_bounds__(kBlock) k_em_beta_reduce(EmDev D) {
     const float4 sum = final_reduce<0>(D.partials, groups_of(D.E), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    if (threadIdx.x == 0 && D.scalars[1].w == 0.0f) {
-        D.scalars[1].y = sum.x / D.scalars[0].x;
-        D.scalars[0].x = sum.x;
-        D.scalars[0].y = sum.y;
-        D.scalars[1].z += 1.0f;
-        if (sum.y <= D.scalars[0].w) D.scalars[1].w = 1.0f;
-        if (fabsf(sum.x) > 3e38f || fabsf(sum.y) > 3e38f) D.scalars[1].w = 2.0f;
-    }
+    if (threadIdx.x == 0) set_beta(D, make_float2(sum.x, sum.y));
 }
 // update_search (induction.wgsl:214): z = r/d, or the nodal z left in w
+template <int N>
 __global__ void __launch_bounds__(kBlock) k_em_update_search(EmDev D) {
-    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i < D.E && active(D)) {
-        const float z = D.nodal ? D.w[i] : D.r[i] / D.w[i];
-        D.p[i] = z + D.scalars[1].y * D.p[i];
+    if (!active(D)) return;
+    const uint32_t base = blockIdx.x * (N * kBlock) + threadIdx.x;
+    const float beta = D.scalars[1].y;
+    float r[N], w[N], pv[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t i = base + k * kBlock;
+        if (i >= D.E) continue;
+        r[k] = D.nodal ? 0.0f : D.r[i];
+        w[k] = D.w[i];
+        pv[k] = D.p[i];
+    }
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t i = base + k * kBlock;
+        if (i < D.E) D.p[i] = (D.nodal ? w[k] : r[k] / w[k]) + beta * pv[k];
     }
 }
 // true_residual (induction.wgsl:230-240)
@@ -1227,14 +1314,26 @@ static void em_append_nodal(mhdproj_em_ctx* ctx, bool initial) {
         EM_LAUNCH(k_em_nodal<false>, D.E, D);
     }
 }
-static void em_iteration(mhdproj_em_ctx* ctx) {
+template <int N>
+static void em_iteration_n(mhdproj_em_ctx* ctx) {
     const EmDev& D = ctx->D;
+    const unsigned blocks = (D.E + N * kBlock - 1) / (N * kBlock);
     EM_LAUNCH(k_em_apply<true>, D.E, D);
     EM_SINGLE(k_em_alpha_reduce, D);
-    EM_LAUNCH(k_em_update_residual, D.E, D);
-    em_append_nodal(ctx, false);
-    EM_SINGLE(k_em_beta_reduce, D);
-    EM_LAUNCH(k_em_update_search, D.E, D);
+    if (D.nodal) {
+        k_em_update_residual<N, false><<<blocks, kBlock, 0, ctx->stream>>>(D);
+        em_append_nodal(ctx, false);
+        EM_SINGLE(k_em_beta_reduce, D);
+    } else {
+        k_em_update_residual<N, true><<<blocks, kBlock, 0, ctx->stream>>>(D);
+        EM_SINGLE(k_em_beta_reduce_pairs, D);
+    }
+    k_em_update_search<N><<<blocks, kBlock, 0, ctx->stream>>>(D);
+    ctx->launches += 2;
+}
+static void em_iteration(mhdproj_em_ctx* ctx) {
+    if (ctx->D.E >= kManyEdges) em_iteration_n<kEdges>(ctx);
+    else em_iteration_n<1>(ctx);
 }
 // The iteration kernels take EmDev by value, so the graph holds the step
 // constants they read (initial, dt, nodal mode); it is captured again when
@@ -1680,7 +1779,7 @@ int mhdproj_em_advance(mhdproj_em_ctx* ctx, double time_s, int initial, const fl
             const uint32_t batch = std::min(cap - its(), kBatch);
             if (batch == kBatch && ctx->batch) {
                 EK(cudaGraphLaunch(ctx->batch, ctx->stream));
-                ctx->launches += 5 * kBatch;
+                ctx->launches += (D.nodal ? 7 : 5) * kBatch;
             } else {
                 for (uint32_t k = 0; k < batch; k++) em_iteration(ctx);
             }
