@@ -660,37 +660,39 @@ __global__ void kr_mg_jacobi(MView m, int temp) {
         else m.value[off + i].z = next;
     }
 }
-// restrict_residual (:74-83)
+// restrict_residual (:74-83).  Eight threads per coarse cell, one child's
+// residual each; the first adds them in the shader's order (a child that the
+// shader skips adds zero, which changes no bit).  One thread per cell was a
+// chain of 8 x 7 dependent neighbourhoods, whose latency set the time even of
+// a single block (15 to 27 us a launch on every level; a projection of the
+// 96^3 jet 14.8 ms, a third of it here).
 __global__ void kr_mg_restrict(MView m) {
     if (mg_converged(m)) return;
     const Level& L = m.L;
-    const uint32_t i = blockIdx.x * WG + threadIdx.x;
-    if (i >= L.dims[3]) return;
-    const I3 q = decode3(i, L.dims);
-    const bool fine = L.location[2] == 1u;
+    const uint32_t t = blockIdx.x * WG + threadIdx.x, i = t >> 3;
+    float own = 0.0f;
+    if (i < L.dims[3]) {
+        const I3 q = decode3(i, L.dims);
+        const bool fine = L.location[2] == 1u;
+        I3 child;
+        child.v[0] = 2 * q.v[0] + (int)(t & 1u);
+        child.v[1] = 2 * q.v[1] + (int)(t >> 1 & 1u);
+        child.v[2] = 2 * q.v[2] + (int)(t >> 2 & 1u);
+        if (mg_valid(child, L.child)) {
+            const uint32_t ci = idx3(child, L.child);
+            if (!fine) own = m.value[L.location[1] + ci].x - mg_action(m, child, L.child, L.location[1], false, false);
+            else if (fine_active(m, ci)) own = m.work[ci].y - mg_action(m, child, L.child, L.location[1], true, false);
+        }
+    }
     float sum = 0.0f;
-    for (int z = 0; z < 2; z++)
-        for (int y = 0; y < 2; y++)
-            for (int x = 0; x < 2; x++) {
-                I3 child;
-                child.v[0] = 2 * q.v[0] + x;
-                child.v[1] = 2 * q.v[1] + y;
-                child.v[2] = 2 * q.v[2] + z;
-                if (!mg_valid(child, L.child)) continue;
-                const uint32_t ci = idx3(child, L.child);
-                float r;
-                if (fine) {
-                    if (!fine_active(m, ci)) continue;
-                    r = m.work[ci].y;
-                } else {
-                    r = m.value[L.location[1] + ci].x;
-                }
-                sum += r - mg_action(m, child, L.child, L.location[1], fine, false);
-            }
-    float4& v = m.value[L.location[0] + i];
-    v.x = sum;
-    v.y = 0.0f;
-    v.z = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) sum += __shfl_sync(0xffffffffu, own, k, 8);
+    if (i < L.dims[3] && (t & 7u) == 0u) {
+        float4& v = m.value[L.location[0] + i];
+        v.x = sum;
+        v.y = 0.0f;
+        v.z = 0.0f;
+    }
 }
 // prolong (:84-88)
 __global__ void kr_mg_prolong(MView m) {
@@ -1096,7 +1098,7 @@ static void mg_cycle(RefState* s) {  // cycle_stages (multigrid.rs:67-82)
     const int L = (int)s->levels.size();
     for (int l = 0; l + 1 < L; l++) {
         kr_mg_diagonal_start<<<blocks_for(s->levels[l].dims[3]), WG, 0, s->stream>>>(mview(s, l));
-        kr_mg_restrict<<<blocks_for(s->levels[l + 1].dims[3]), WG, 0, s->stream>>>(mview(s, l + 1));
+        kr_mg_restrict<<<blocks_for(8 * s->levels[l + 1].dims[3]), WG, 0, s->stream>>>(mview(s, l + 1));
     }
     kr_mg_coarse_solve<<<1, WG, 0, s->stream>>>(mview(s, L - 1));
     for (int l = L - 2; l >= 0; l--) {

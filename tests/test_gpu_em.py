@@ -376,3 +376,18 @@ def test_energy_ledger_bit_exact(gpu):
         scale = abs(g["external_j"]) + abs(g["delta_magnetic_j"]) + g["joule_j"] + g["backward_euler_j"]
         assert abs(g["balance_error_j"]) / scale < 1e-4
     pair.close()
+
+
+@pytest.mark.parametrize("n,after", [(47, 1024), (48, 16)])
+def test_many_edges_bit_exact(gpu, n, after):
+    """Enough edges for the passes that take several edges a thread, with
+    remainders of whole and of part groups (47: 324864 edges, 48: 345744), and
+    without and with the nodal correction."""
+    import mhdproj
+
+    pair, applied = _driven_pair(gpu, mhdproj, n, nodal_switch_after=after)
+    pair.set_materials()
+    pair.step(0.0, initial=True, applied=applied(0.0), label="initial")
+    _, st, _ = pair.step(1e-5, applied=applied(1e-5), label="step")
+    assert st[7] == 1.0
+    pair.close()
