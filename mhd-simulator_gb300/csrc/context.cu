@@ -857,17 +857,19 @@ static void begin_scalars(mhdproj_ctx* ctx, bool adjoint = false) {
     // against 3.5e-6 with two), so with them on every level above the bottom
     // sub-cycle a pass aims at 1/16 (4e-7; about one iteration more), and
     // where other levels lie between, whose two half-steps leave rougher
-    // residuals, at 1/8.  An adjoint's right-hand side has more weight on
-    // smooth modes, whose error a residual shows least: a quarter of that (vjp
-    // jet 192x160x132: 4e-6 off FP64 at 1/16, 1e-7 at 1/64, 7e-7 with two
-    // half-steps at half the tolerance).
+    // residuals, at 1/8.An adjoint's right-hand side has more weight on
+    // smooth modes, and its goal lies close to the reduction that a pass stops
+    // at: a restart there loses what CG knows of those modes, so it runs on to
+    // the goal itself where FP32 lets it (vjp jet 192x160x132: 4.75 ms and 3e-7
+    // off FP64; with the restart 5.9 ms and 1.6e-6; two half-steps 6.3 ms and
+    // 7e-7).
     const MGPlan& P = ctx->mg;
-    double pass_margin = 1.0 / 4;
+    double pass_margin = 1.0 / 4, inner_floor2 = 1e-10;
     if (ctx->pipelined && P.lv[0].passes != PASS_PAIR) {
         pass_margin = P.bottom_from > 0 && P.fused_levels >= P.bottom_from ? 1.0 / 256 : 1.0 / 64;
-        if (adjoint) pass_margin /= 16;
+        if (adjoint) inner_floor2 = 1e-13;
     }
-    launch_init_scalars(ctx->sc, tol2, abs_floor, 1e-10, pass_margin, (int)ctx->opt.max_iterations, ctx->stream);
+    launch_init_scalars(ctx->sc, tol2, abs_floor, inner_floor2, pass_margin, (int)ctx->opt.max_iterations, ctx->stream);
 }
 
 static const char* const MEANFREE_ADJOINT =
