@@ -606,17 +606,20 @@ static Launch pair_launch(const Launch& L, int occ_kind) {
     const int gx = (L.g.nx + PX - 1) / PX, gy = (L.g.ny + TY - 1) / TY, nz = L.g.nz;
     const int tiles = gx * gy;
     const int cap = (g_sms > 0 ? g_sms : 152) * (g_occ[occ_kind] > 0 ? g_occ[occ_kind] : 2);
-    // candidate even z runs of at least 8 planes (or the whole column):
-    // pick the one whose grid wastes the least of its last wave
+    // candidate even z runs of at least 8 planes (or the whole column), and
+    // shorter ones while the grid stays within one wave, where the length of a
+    // block's march sets the time (30x22x17: 6 blocks before; 1214 us a
+    // projection, 939 now): pick the one whose grid wastes the least of its
+    // last wave
     int best_zper = nz, best_zc = 1;
     double best = -1.0;
     for (int zc = 1; zc <= nz; zc++) {
         int zper = (nz + zc - 1) / zc;
         if ((zper & 1) && zper < nz) zper++;
-        if (zper < 8 && zc > 1) break;
+        if (zper < 2 && zc > 1) break;
         const int zcr = (nz + zper - 1) / zper;
         const long long blocks = (long long)tiles * zcr;
-        if (blocks > MAX_REDUCE_BLOCKS) break;
+        if (blocks > MAX_REDUCE_BLOCKS || (zper < 8 && zc > 1 && blocks > cap)) break;
         const double waves = (double)blocks / cap;
         // fullness of the last wave times the share of fetched planes that
         // are computed (each run also fetches the planes just below and above)
