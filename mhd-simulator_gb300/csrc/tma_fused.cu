@@ -122,7 +122,7 @@ struct PassSm {
     alignas(128) ET c[G::NS][G::RH][RS];
     // the three stages' half-planes, each for the next step (slot: step & 1)
     alignas(16) float ex[3][2][G::RH][HH];
-    float4 ypart[G::FTY / 2][QO];  // restriction sums of the odd rows
+    float4 ypart[2][G::FTY / 2][QO];  // restriction sums of the odd rows (slot: rc_slot)
     unsigned long long bar[2];
     int abort_;
 };
@@ -310,6 +310,30 @@ struct RecordRing {
     }
 };
 
+// Restriction sums of a run of planes z0 .. z1-1: in step k, whose output stage
+// works on plane zC = z0 + k - 6, a coarse plane's sums are complete after its odd
+// plane or the run's last one.  The odd rows' threads leave theirs in shared
+// memory late in that step and the even rows' take them at the start of the next
+// one.  With an odd number of planes the last two steps of a run each complete a
+// coarse plane, so a step may leave one while it takes another: two slots, by the
+// coarse plane's parity.
+constexpr bool rc_complete(int k, int zC, int z1) { return k >= 6 && ((zC & 1) || zC + 1 == z1); }
+__host__ __device__ constexpr int rc_slot(int zc) { return zc & 1; }
+// No step of a run takes from the slot that it leaves sums in (one barrier
+// separates two steps, none the ends of one).
+constexpr bool rc_exchange_ordered() {
+    for (int n = 1; n <= 9; n++) {  // planes of a run from z0 = 0
+        int pending = -1;
+        for (int k = 0; k < n + 6; k++) {
+            const int taken = pending;
+            pending = rc_complete(k, k - 6, n) ? rc_slot((k - 6) >> 1) : -1;
+            if (pending >= 0 && pending == taken) return false;
+        }
+    }
+    return true;
+}
+static_assert(rc_exchange_ordered(), "a slot of restriction sums is overwritten in the step that reads it");
+
 // ---------------------------------------------------------------- down pass
 // rin (VT) -> the black half of the correction (compact rows) and the coarse
 // residual rc.  UPDATE (finest level inside CG): r_out = rin - alpha q is
@@ -371,7 +395,7 @@ __global__ void __launch_bounds__(OGeo<CK>::NT, 1)
     int rc_z = -1;  // coarse plane of ph
     auto flush_rc = [&]() {
         if (rc_z >= 0 && own_warp && !(gy & 1)) {
-            const float4 o = S.ypart[(T.row - 3) >> 1][T.oc - 1];
+            const float4 o = S.ypart[rc_slot(rc_z)][(T.row - 3) >> 1][T.oc - 1];
             VTc* cp = rc + ((gx >> 1) + (long long)gc.nx * ((gy >> 1) + (long long)gc.ny * rc_z));
             if (in_a) st2<VTc>(cp, make_float2(0.25f * (ph[0] + o.x), 0.25f * (ph[1] + o.y)));
             if (in_b) st2<VTc>(cp + 2, make_float2(0.25f * (ph[2] + o.z), 0.25f * (ph[3] + o.w)));
@@ -449,14 +473,13 @@ __global__ void __launch_bounds__(OGeo<CK>::NT, 1)
 #pragma unroll
                     for (int j = 0; j < 4; j++) pa[j] += acc[j];
                 }
-                if (k >= 5 && ((zC & 1) || zC + 1 == z1)) {
-                    // the pair's sums are complete (at k = 5 planes z0 and z0+1 become
-                    // the first pair)
-                    if (k >= 6) {
-                        if (gy & 1) put4(&S.ypart[(T.row - 3) >> 1][T.oc - 1].x, pa);
-                        copy4(ph, pa);
-                        rc_z = zC >> 1;
-                    }
+                const bool complete = rc_complete(k, zC, z1);
+                if (complete) {
+                    if (gy & 1) put4(&S.ypart[rc_slot(zC >> 1)][(T.row - 3) >> 1][T.oc - 1].x, pa);
+                    copy4(ph, pa);
+                    rc_z = zC >> 1;
+                }
+                if (complete || k == 5) {  // at k = 5 planes z0 and z0+1 become the first pair
                     copy4(pa, pb);
 #pragma unroll
                     for (int j = 0; j < 4; j++) pb[j] = 0.f;
