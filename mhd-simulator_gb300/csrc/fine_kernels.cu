@@ -86,8 +86,8 @@ struct Fetcher {
             if (k < NE) {
                 const int ty = k / EP, pi = k - ty * EP;
                 bool okx, oky;
-                const int sx = axis_src(x0 - 2 + 2 * pi, g.nx, px, &okx);
-                const int sy = axis_src(y0 - 1 + ty, g.ny, py, &oky);
+                const int sx = axis_wrap(x0 - 2 + 2 * pi, g.nx, px, &okx);
+                const int sy = axis_wrap(y0 - 1 + ty, g.ny, py, &oky);
                 eok[j] = okx && oky;
                 eoff[j] = eok[j] ? sx + g.nx * sy : 0;
                 edst[j] = (short)(ty * EW + 2 * pi);
@@ -104,8 +104,8 @@ struct Fetcher {
                 const int ty = k / CPR, ci = k - ty * CPR;
                 const int cx = (CK == 0) ? ci : (ci < TX ? 2 * ci : PX);
                 bool okx, oky;
-                const int sx = axis_src(x0 + cx, g.nx, px, &okx);
-                const int sy = axis_src(y0 + ty, g.ny, py, &oky);
+                const int sx = axis_wrap(x0 + cx, g.nx, px, &okx);
+                const int sy = axis_wrap(y0 + ty, g.ny, py, &oky);
                 cok[j] = okx && oky;
                 coff[j] = cok[j] ? sx + g.nx * sy : 0;
                 cdst[j] = (short)(ty * CW + cx);
@@ -121,7 +121,7 @@ struct Fetcher {
     __device__ __forceinline__ void fetch(Ring<CK>& R, int zz, int slot, const float* ev,
                                           const typename CoefStore<CK>::T* coef, const float* rv) const {
         bool okz;
-        const int sz = axis_src(zz, nz, pz, &okz);
+        const int sz = axis_wrap(zz, nz, pz, &okz);
         const long long plane = (long long)sz * sxy;
         if (WANT_E) {
             float* dst = &R.e[slot][0][0];
@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_search_spmv(Grid3 g, const flo
     if (t < NSV) {
         const int row = t / SG, gi = t - row * SG;
         bool okx, oky;
-        const int sx = axis_src(x0 - 4 + 4 * gi, g.nx, px, &okx);
-        const int sy = axis_src(y0 - 1 + row, g.ny, py, &oky);
+        const int sx = axis_wrap(x0 - 4 + 4 * gi, g.nx, px, &okx);
+        const int sy = axis_wrap(y0 - 1 + row, g.ny, py, &oky);
         vok = okx && oky;
         voff = vok ? sx + g.nx * sy : 0;
         vdst = (short)(row * SW + 4 * gi);
@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_search_spmv(Grid3 g, const flo
         if (k < NSC) {
             const int row = k / (PX + 1), cx = k - row * (PX + 1);
             bool okx, oky;
-            const int sx = axis_src(x0 + cx, g.nx, px, &okx);
-            const int sy = axis_src(y0 + row, g.ny, py, &oky);
+            const int sx = axis_wrap(x0 + cx, g.nx, px, &okx);
+            const int sy = axis_wrap(y0 + row, g.ny, py, &oky);
             cok[u] = okx && oky;
             coff[u] = cok[u] ? sx + g.nx * sy : 0;
             cdst[u] = (short)(row * CW + cx);
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_search_spmv(Grid3 g, const flo
     }
     auto fetch = [&](int zz, int s2, int s4) {
         bool okz;
-        const int sz = axis_src(zz, g.nz, pz, &okz);
+        const int sz = axis_wrap(zz, g.nz, pz, &okz);
         const long long plane = (long long)sz * sxy;
         if (vdst >= 0) {
             const bool ok = vok && okz;

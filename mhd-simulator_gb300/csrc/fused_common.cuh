@@ -80,15 +80,6 @@ template <> __device__ __forceinline__ void st2<__nv_bfloat16>(__nv_bfloat16* p,
     *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v.x, v.y);
 }
 
-// Wrapped or absent coordinate along one axis, any number of periods away (a
-// halo or the rest of a tile can be wider than the grid).
-__device__ __forceinline__ int axis_wrap(int c, int n, bool periodic, bool* ok) {
-    *ok = periodic || (c >= 0 && c < n);
-    if (c < 0) return periodic ? n - 1 - (-1 - c) % n : 0;
-    if (c >= n) return periodic ? c % n : n - 1;
-    return c;
-}
-
 // The smoother records in HBM are split along whole grid rows: row (y, z)
 // holds its nx/2 even-x records, then its nx/2 odd-x records.  Position of
 // column x in its row:

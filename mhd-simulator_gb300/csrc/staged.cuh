@@ -54,19 +54,27 @@ template <> __device__ __forceinline__ float4 unpack<2>(const uint2& u) {
     return make_float4(fa.x, fa.y, fb.x, fb.y);
 }
 
-// Wrapped or absent coordinate along one axis.
-__device__ __forceinline__ int axis_src(int c, int n, bool periodic, bool* ok) {
-    if (c < 0) {
-        *ok = periodic;
-        return periodic ? c + n : 0;
-    }
-    if (c >= n) {
-        *ok = periodic;
-        return periodic ? c - n : n - 1;
-    }
-    *ok = true;
+// Wrapped or absent coordinate along one axis, any number of periods away (a
+// halo or the rest of a tile can be wider than the grid).
+__host__ __device__ constexpr int axis_wrap(int c, int n, bool periodic, bool* ok) {
+    *ok = periodic || (c >= 0 && c < n);
+    if (c < 0) return periodic ? n - 1 - (-1 - c) % n : 0;
+    if (c >= n) return periodic ? c % n : n - 1;
     return c;
 }
+// Every coordinate that a tile of 64 columns or 32 rows with its halo reaches
+// lands inside the grid, on a periodic axis a whole number of periods away.
+constexpr bool axis_wrap_in_range() {
+    for (int n = 1; n <= 72; n++)
+        for (int c = -8; c < n + 72; c++)
+            for (int periodic = 0; periodic < 2; periodic++) {
+                bool ok = false;
+                const int w = axis_wrap(c, n, periodic != 0, &ok);
+                if (w < 0 || w >= n || ok != (periodic || (c >= 0 && c < n)) || (ok && (c - w) % n != 0)) return false;
+            }
+    return true;
+}
+static_assert(axis_wrap_in_range(), "a wrapped coordinate leaves the grid");
 
 // Rotating slot indices of the plane rings: index of plane zA + k.
 struct Slots {

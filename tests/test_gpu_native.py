@@ -462,3 +462,35 @@ def test_mean_free_gauge_refuses_the_adjoint(gpu):
     pinned = make(mhdproj, c, precision="fp16", rel_tol=1e-6, gauge=0)
     pinned.set_coefficients(a, s, c["rho_liquid"], c["rho_air"])
     pinned.vjp(us, None, c["dt"])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+@pytest.mark.parametrize("dims,periodic", [((16, 12, 10), 3), ((20, 4, 18), 3), ((32, 2, 6), 2), ((8, 6, 2), 7), ((18, 6, 8), 3), ((2, 4, 2), 7)],
+                         ids=str)
+def test_projection_on_periodic_grids_narrower_than_a_tile(gpu, oracle_lib, dims, periodic, precision):
+    """A tile of 64 x 8 cells with its halo reaches past these grids by more
+    than one period (18, 2: the staged kernels of cell pairs; the others the
+    fused passes)."""
+    import mhdproj
+
+    torch = gpu
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nx + ny + nz)
+    alpha = (0.5 + 0.45 * np.sin(rng.uniform(0, 6.0, (nz, ny, nx)))).astype(np.float32)
+    us = [rng.standard_normal(s).astype(np.float32) for s in ((nz, ny, nx + 1), (nz, ny + 1, nx), (nz + 1, ny, nx))]
+    for a, v in enumerate(us):  # a periodic axis repeats its first face, a wall's is 0
+        first, last = v.swapaxes(2 - a, 0)[0], v.swapaxes(2 - a, 0)[-1]
+        if not periodic >> a & 1:
+            first[...] = 0.0
+        last[...] = first
+    c = dict(dims=dims, h=1e-3, periodic=periodic, outlet=False, rho_liquid=1000.0, rho_air=10.0, alpha=alpha,
+             solid=np.zeros((nz, ny, nx), np.uint8), u=us[0], v=us[1], w=us[2], dt=1e-4)
+    pr = make(mhdproj, c, precision=precision, rel_tol=1e-8)
+    a, s, ut = tensors(torch, c)
+    pr.set_coefficients(a, s, c["rho_liquid"], c["rho_air"])
+    out, p, st = pr.project(ut, c["dt"])
+    assert st.true_relative_residual <= 1e-8
+    ref = oracle_lib.project(ogrid(oracle_lib, c), alpha, c["solid"], *us, c["dt"], 1e-13)
+    for o, k in zip(out, "uvw"):
+        assert rel_l2(o.cpu().numpy(), ref[k]) < 1e-5
+    assert rel_l2(p.cpu().numpy(), ref["p"]) < 1e-5
