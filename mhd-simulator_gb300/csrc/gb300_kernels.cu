@@ -868,37 +868,33 @@ __global__ void __launch_bounds__(TILE_THREADS) k_adj_correct(Grid3 g, int outle
     }
 }
 
-// The force terms of a chain step, dt f / rho with the exact face density, to
-// double-FP32 (error below 2^-45) instead of FP64, whose divisions bound these
-// passes: 128^3, k_add_force 338 us, k_force_grad 169 us with them (a chain of
-// eight steps and its gradient: 46.7 ms, 43.1 ms without).  Products
-// outside the range in which both words are normal numbers take the FP64 form,
-// infinities and NaN among them.
-__device__ __forceinline__ df face_rho(float aL, float aR, float rho_l, float rho_air) {
-    return two_sum(0.5f * rho_of(aL, rho_l, rho_air), 0.5f * rho_of(aR, rho_l, rho_air));
-}
-__device__ __forceinline__ df cell_rho(float a, float rho_l, float rho_air) { return {rho_of(a, rho_l, rho_air), 0.0f}; }
-__device__ __forceinline__ double df_to_d(df a) { return (double)a.hi + (double)a.lo; }
-__device__ __forceinline__ bool df_range(df p) { return fabsf(p.hi) > 1e-25f && fabsf(p.hi) < 1e30f; }
-__device__ __forceinline__ df df_div(df a, df b) {
-    const float q = __fdiv_rn(a.hi, b.hi);
-    const df p = two_prod(q, b.hi);
-    const float rest = __fmaf_rn(-q, b.lo, __fadd_rn(__fsub_rn(__fsub_rn(a.hi, p.hi), p.lo), a.lo));
-    return fast_two_sum(q, __fdiv_rn(rest, b.hi));
-}
-// u + dt f / rho
-__device__ __forceinline__ float add_force(float u, float f, float dt, df rho) {
-    const df p = two_prod(dt, f);
-    if (df_range(p)) return df_to_f(df_add_f(df_div(p, rho), u));
-    if (f == 0.0f && dt < 1e30f) return u + p.hi;
-    return (float)((double)u + (double)dt * (double)f / df_to_d(rho));
-}
-// dt / rho * lambda
-__device__ __forceinline__ double force_grad(float dt, float lambda, df rho) {
-    const df p = two_prod(dt, lambda);
-    if (df_range(p)) return df_to_d(df_div(p, rho));
-    if (lambda == 0.0f && dt < 1e30f) return p.hi;
-    return (double)dt / df_to_d(rho) * (double)lambda;
+// The force terms of a chain step: dt f / rho with the exact face density, in
+// FP64, whose divisions bound such a pass (128^3: k_force_grad 169 us).  The
+// velocity is rounded to FP32, so k_add_force first forms it in double-FP32 and
+// asks whether every value within that form's error rounds to the same FP32
+// number (Ziv's rounding test, 1991); the one face in some 30 thousand where it
+// does not, and infinities, NaN and quotients out of the range of normal pairs,
+// take FP64.  The same bits either way, 48 us instead of 338.  The gradient is
+// summed in FP64, for which a pair is too short.
+__device__ __forceinline__ double face_rho(float rL, float rR) { return 0.5 * ((double)rL + (double)rR); }
+// u + dt f / rho, rho the mean of rL and rR
+__device__ __forceinline__ float add_force(float u, float f, float dt, float rL, float rR) {
+    const df rho = two_sum(0.5f * rL, 0.5f * rR), p = two_prod(dt, f);
+    if (f == 0.0f && dt < 1e30f && rho.hi > 0.0f) return u + p.hi;
+    if (fabsf(p.hi) > 1e-25f && fabsf(rho.hi) > 1e-30f) {
+        // q = p / rho, |error| < 2^-44 |q|, or 1e-43 where a word is subnormal
+        const float q = __fdiv_rn(p.hi, rho.hi);
+        const df t = two_prod(q, rho.hi);
+        const float ql =
+            __fdiv_rn(__fmaf_rn(-q, rho.lo, __fadd_rn(__fsub_rn(__fsub_rn(p.hi, t.hi), t.lo), p.lo)), rho.hi);
+        // u + q = s.hi + lo, |error| < 2^-42 (|u| + |q|) more
+        const df s = two_sum(q, u);
+        const float lo = __fadd_rn(s.lo, ql);
+        const float err = __fmaf_rn(0x1p-40f, __fadd_rn(fabsf(u), fabsf(q)), 1e-40f);
+        const float a = __fadd_rn(s.hi, __fsub_rn(lo, err)), b = __fadd_rn(s.hi, __fadd_rn(lo, err));
+        if (a == b && fabsf(a) < 1e38f) return a;
+    }
+    return (float)((double)u + (double)dt * (double)f / face_rho(rL, rR));
 }
 // u* = u + dt f / rho_face on open faces (closed faces copied through).
 __global__ void __launch_bounds__(TILE_THREADS) k_add_force(Grid3 g, int outlet, float rho_l, float rho_air,
@@ -919,7 +915,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_add_force(Grid3 g, int outlet,
             const int f = x + (nx + 1) * (y + ny * z);
             float out = u[f];
             if (nb.xm >= 0 && ci != 0 && cls[nb.xm] != 0)
-                out = add_force(u[f], fu[f], dt, face_rho(alpha[nb.xm], alpha[i], rho_l, rho_air));
+                out = add_force(u[f], fu[f], dt, rho_of(alpha[nb.xm], rho_l, rho_air),
+                                rho_of(alpha[i], rho_l, rho_air));
             su[f] = out;
             if (x == nx - 1) su[nx + (nx + 1) * (y + ny * z)] = u[nx + (nx + 1) * (y + ny * z)];
         }
@@ -927,7 +924,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_add_force(Grid3 g, int outlet,
             const int f = x + nx * (y + (ny + 1) * z);
             float out = v[f];
             if (nb.ym >= 0 && ci != 0 && cls[nb.ym] != 0)
-                out = add_force(v[f], fv[f], dt, face_rho(alpha[nb.ym], alpha[i], rho_l, rho_air));
+                out = add_force(v[f], fv[f], dt, rho_of(alpha[nb.ym], rho_l, rho_air),
+                                rho_of(alpha[i], rho_l, rho_air));
             sv[f] = out;
             if (y == ny - 1) sv[x + nx * (ny + (ny + 1) * z)] = v[x + nx * (ny + (ny + 1) * z)];
         }
@@ -935,13 +933,14 @@ __global__ void __launch_bounds__(TILE_THREADS) k_add_force(Grid3 g, int outlet,
             const int f = x + nx * (y + ny * z);
             float out = w[f];
             if (nb.zm >= 0 && ci != 0 && cls[nb.zm] != 0)
-                out = add_force(w[f], fw[f], dt, face_rho(alpha[nb.zm], alpha[i], rho_l, rho_air));
+                out = add_force(w[f], fw[f], dt, rho_of(alpha[nb.zm], rho_l, rho_air),
+                                rho_of(alpha[i], rho_l, rho_air));
             sw[f] = out;
             if (z == nz - 1) {
                 const int ft = x + nx * (y + ny * nz);
                 float top = w[ft];
                 if (outlet && !(g.periodic & 4) && ci != 0)
-                    top = add_force(w[ft], fw[ft], dt, cell_rho(alpha[i], rho_l, rho_air));
+                    top = add_force(w[ft], fw[ft], dt, rho_of(alpha[i], rho_l, rho_air), rho_of(alpha[i], rho_l, rho_air));
                 sw[ft] = top;
             }
         }
@@ -957,6 +956,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_force_grad(Grid3 g, int outlet
                                                              double* __restrict__ gu, double* __restrict__ gv,
                                                              double* __restrict__ gw) {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const double dtd = (double)dt;
     TILE_BEGIN(g) {
         if (!in_xy) continue;
         const int i = cell_index(g, x, y, z);
@@ -964,19 +964,19 @@ __global__ void __launch_bounds__(TILE_THREADS) k_force_grad(Grid3 g, int outlet
         const uint8_t ci = cls[i];
         if (nb.xm >= 0 && ci != 0 && cls[nb.xm] != 0) {
             const int f = x + (nx + 1) * (y + ny * z);
-            gu[f] += force_grad(dt, lu[f], face_rho(alpha[nb.xm], alpha[i], rho_l, rho_air));
+            gu[f] += dtd / face_rho(rho_of(alpha[nb.xm], rho_l, rho_air), rho_of(alpha[i], rho_l, rho_air)) * (double)lu[f];
         }
         if (nb.ym >= 0 && ci != 0 && cls[nb.ym] != 0) {
             const int f = x + nx * (y + (ny + 1) * z);
-            gv[f] += force_grad(dt, lv[f], face_rho(alpha[nb.ym], alpha[i], rho_l, rho_air));
+            gv[f] += dtd / face_rho(rho_of(alpha[nb.ym], rho_l, rho_air), rho_of(alpha[i], rho_l, rho_air)) * (double)lv[f];
         }
         if (nb.zm >= 0 && ci != 0 && cls[nb.zm] != 0) {
             const int f = x + nx * (y + ny * z);
-            gw[f] += force_grad(dt, lw[f], face_rho(alpha[nb.zm], alpha[i], rho_l, rho_air));
+            gw[f] += dtd / face_rho(rho_of(alpha[nb.zm], rho_l, rho_air), rho_of(alpha[i], rho_l, rho_air)) * (double)lw[f];
         }
         if (z == nz - 1 && outlet && !(g.periodic & 4) && ci != 0) {
             const int ft = x + nx * (y + ny * nz);
-            gw[ft] += force_grad(dt, lw[ft], cell_rho(alpha[i], rho_l, rho_air));
+            gw[ft] += dtd / (double)rho_of(alpha[i], rho_l, rho_air) * (double)lw[ft];
         }
     }
 }

@@ -494,3 +494,39 @@ def test_projection_on_periodic_grids_narrower_than_a_tile(gpu, oracle_lib, dims
     for o, k in zip(out, "uvw"):
         assert rel_l2(o.cpu().numpy(), ref[k]) < 1e-5
     assert rel_l2(p.cpu().numpy(), ref["p"]) < 1e-5
+
+
+def test_chain_force_equals_the_fp64_form(gpu):
+    """u + dt f / rho in FP64, rounded to FP32, bit for bit.  With velocity,
+    force and density constant along a periodic x axis the sum has no
+    divergence, so a step returns it as it is.  Sums next to a rounding
+    boundary of FP32 (quotients of odd half units in the last place), of any
+    exponents, products outside the range of normal pairs, zeros."""
+    import mhdproj
+
+    torch = gpu
+    nx, ny, nz = 8, 64, 128
+    m = ny * nz // 4
+    rng = np.random.default_rng(11)
+    f32, dt, rl, ra = np.float32, np.float32(1e-6), np.float32(6440.0), np.float32(1.2)
+    a = rng.random(ny * nz, f32)
+    a[::7], a[3::7] = 1.0, 0.0
+    rho = (ra * (f32(1) - a) + rl * a).astype(np.float64)
+    sign = lambda k: rng.choice([-1.0, 1.0], k)
+    power = lambda k, lo, hi: sign(k) * 2.0 ** rng.uniform(lo, hi, k)
+    u = np.concatenate([rng.uniform(0.5, 1.5, m) * sign(m), power(m, -90, 60), power(m, -20, 20), rng.choice([0.0, -0.0, 1.0, -3e-5], m)]).astype(f32)
+    q = np.concatenate([np.spacing(np.abs(u[:m])).astype(np.float64) * (rng.integers(-4, 4, m) + 0.5), power(m, -90, 60),
+                        power(m, -80, 20), power(m, -110, -70) * rng.choice([0.0, 1.0], m)])
+    f = (q * rho / np.float64(dt)).astype(f32)
+    want = (u.astype(np.float64) + np.float64(dt) * f.astype(np.float64) / rho).astype(f32)
+    assert np.isfinite(want).all() and (want != u).sum() > m
+    t = lambda v: torch.from_numpy(np.ascontiguousarray(np.broadcast_to(v.reshape(nz, ny, 1), (nz, ny, nx + 1)))).cuda()
+    zero = [torch.zeros((nz, ny + 1, nx), device="cuda"), torch.zeros((nz + 1, ny, nx), device="cuda")]
+    pr = mhdproj.PressureProjection((nx, ny, nz), 1e-4, periodic=[True] * 3, outlet=False, gauge=0)
+    pr.set_coefficients(t(a)[:, :, :nx].contiguous(), torch.zeros((nz, ny, nx), dtype=torch.uint8, device="cuda"), float(rl), float(ra))
+    (ux, _, _), _, st = pr.chain_forward([t(u), *zero], [t(f), *zero], float(dt), 1, 1)
+    assert st.iterations == 0
+    got = ux.cpu().numpy()
+    pr.close()
+    assert np.array_equal(got[:, :, 0], want.reshape(nz, ny)) and np.array_equal(got[:, :, -1], got[:, :, 0])
+    assert np.array_equal(got[:, :, 3], got[:, :, 0])
