@@ -35,6 +35,8 @@ struct Scalars {
     double tol2;        // relative tolerance squared
     double inner_floor2;// minimum inner relative reduction squared
     double pass_margin; // share of the goal on ||r||^2 that a pass aims at
+    double accept_short;// share of it with which a pass cut short counts as done
+    double accept;      // the share that ends the present pass
     double objective;   // chain objective / misc reductions
     double divmax, div2;// divergence statistics
     float alpha_f, beta_f, sigma, inv_sigma;

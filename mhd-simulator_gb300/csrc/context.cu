@@ -760,7 +760,6 @@ static int launch_iterations(mhdproj_ctx* ctx, int count) {
 static int solve(mhdproj_ctx* ctx, float* x_hi, float* x_lo, mhdproj_stats* st, bool x_zero = false) {
     Fields F = fields(ctx);
     const double tol2 = (double)ctx->opt.rel_tol * ctx->opt.rel_tol;
-    (void)tol2;
     int passes = 0;
     // x_zero: the right-hand-side kernel already set up the first pass (r = b)
     if (!x_zero) launch_residual(ctx->L, F, x_hi, x_lo, ctx->stream);
@@ -775,6 +774,7 @@ static int solve(mhdproj_ctx* ctx, float* x_hi, float* x_lo, mhdproj_stats* st, 
         if (S.nonfinite) return fail(ctx, MHDPROJ_ERR_NONFINITE, "Nonfinite fluid pressure residual");
         if (S.outer_done) break;
         if (passes > ctx->opt.max_refinements || (uint32_t)S.total_iterations >= max_it) {
+            if (S.rr_true <= tol2 * S.bb + S.abs_floor) break;  // met, if with less margin than a pass aims at
             const double rel = S.bb > 0 ? std::sqrt(S.rr_true / S.bb) : 0.0;
             const double floor_ = ctx->opt.abs_div_tol;
             return fail(ctx, MHDPROJ_ERR_NOT_CONVERGED,
@@ -850,26 +850,31 @@ static void begin_scalars(mhdproj_ctx* ctx, bool adjoint = false) {
     const double tol2 = (double)ctx->opt.rel_tol * ctx->opt.rel_tol;
     const double h = ctx->grid.h;
     const double abs_floor = (double)ctx->opt.abs_div_tol * ctx->opt.abs_div_tol * h * h * h * h * (double)ctx->n_active;
-    // FP32 CG reduces its own residual by about 1e-5 reliably; refine beyond.
-    // A pass aims at half the tolerance on ||r||.  Three half-steps of smoothing
-    // leave a smoother residual than two, whose error is larger at the same
-    // norm (cylinder 64^3 at half the tolerance: pressure 1.2e-5 off FP64,
-    // against 3.5e-6 with two), so with them on every level above the bottom
-    // sub-cycle a pass aims at 1/16 (4e-7; about one iteration more), and
-    // where other levels lie between, whose two half-steps leave rougher
-    // residuals, at 1/8.An adjoint's right-hand side has more weight on
-    // smooth modes, and its goal lies close to the reduction that a pass stops
-    // at: a restart there loses what CG knows of those modes, so it runs on to
-    // the goal itself where FP32 lets it (vjp jet 192x160x132: 4.75 ms and 3e-7
-    // off FP64; with the restart 5.9 ms and 1.6e-6; two half-steps 6.3 ms and
-    // 7e-7).
+    // FP32 CG reduces its own residual by 1e-5 reliably; refine beyond.  The
+    // per-level smoother aims at half the tolerance on ||r||.  The fused passes
+    // with three half-steps leave a smoother residual: at the same norm the error
+    // is larger, and an isolated slow mode (the liquid inside the jet's nozzle) can
+    // sit below the tolerance in the residual but not in the pressure.  Their passes
+    // aim at 1/32, at 1/8 where the finest level runs two half-steps (large FP32
+    // grids), and the first one goes on to 4.9e-6, which finds such a mode before
+    // the restart forgets the search space.  Relative L2 errors of the pressure
+    // at 1e-6 off a solve to 1e-11, jet 256^3 FP16 / BF16 / FP32 (and ms):
+    //   two half-steps, half the tolerance     8.9e-8 1.4e-6 7.7e-8 (11.3 11.4 14.0)
+    //   first pass 1e-5, aim 1/16              3.0e-7 2.0e-6 -      ( 8.5  9.2 -)
+    //   first pass 1e-5, aim 1/32 (FP32 1/8)   3.0e-7 8.0e-9 9.4e-8 ( 9.1 12.9 15.5)
+    //   first pass 4.9e-6, aim 1/32 (FP32 1/8) 8.7e-8 1.7e-8 5.0e-8 ( 8.7 12.0 14.9)
+    // 4.9e-6 is half of the smallest tolerance that a single pass serves.
+    // An adjoint's right-hand side has more weight on smooth modes, and its goal
+    // lies close to the reduction that a pass stops at: its first pass runs on to
+    // 1e-7.  vjp jet 128^3 BF16, three seeds: 8.1e-7 5.1e-7 4.3e-6 with two
+    // half-steps, 6.0e-7 2.3e-4 4.4e-7 to 3e-7 with an aim of 1/16, 1.9e-7 2.2e-7
+    // 2.1e-7 now; 192x160x132 FP16: 5.2 ms and 6.2e-7, 3.4 and 2.4e-6, 4.5 and
+    // 2.7e-7.
     const MGPlan& P = ctx->mg;
-    double pass_margin = 1.0 / 4, inner_floor2 = 1e-10;
-    if (ctx->pipelined && P.lv[0].passes != PASS_PAIR) {
-        pass_margin = P.bottom_from > 0 && P.fused_levels >= P.bottom_from ? 1.0 / 256 : 1.0 / 64;
-        if (adjoint) inner_floor2 = 1e-13;
-    }
-    launch_init_scalars(ctx->sc, tol2, abs_floor, inner_floor2, pass_margin, (int)ctx->opt.max_iterations, ctx->stream);
+    PassGoals goals = {1.0 / 4, 1e-10, 1.0};
+    if (ctx->pipelined)
+        goals = {P.lv[0].passes == PASS_PAIR ? 1.0 / 64 : 1.0 / 1024, adjoint ? 1e-14 : 2.4e-11, 1.0 / 16};
+    launch_init_scalars(ctx->sc, tol2, abs_floor, goals, (int)ctx->opt.max_iterations, ctx->stream);
 }
 
 static const char* const MEANFREE_ADJOINT =

@@ -34,7 +34,13 @@ struct Fields {
 
 // ---- GB300 solver kernels (gb300_kernels.cu)
 void launch_coefficients(const Launch& L, const Fields& F, cudaStream_t s);
-void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, double inner_floor2, double pass_margin, int max_total,
+// Goals of a CG pass, as squares of norms: the share of the tolerance it aims
+// at, the reduction it stops at, and the share of the tolerance with which a
+// pass that stopped at that reduction is accepted (1: any).
+struct PassGoals {
+    double margin, floor2, accept_short;
+};
+void launch_init_scalars(Scalars* sc, double tol2, double abs_floor, const PassGoals& goals, int max_total,
                          cudaStream_t s);
 // start_pass: also r = b, x = 0 and the first pass's scalars (a solve from x = 0)
 void launch_rhs(const Launch& L, const Fields& F, const float* u, const float* v, const float* w, cudaStream_t s,

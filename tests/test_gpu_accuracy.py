@@ -1,0 +1,88 @@
+"""Errors of solves at their tolerance.  The stopping rules look at the norm of
+the residual, which says little about an isolated smooth mode, so the errors
+themselves are held: against a solve to 1e-11 they stay at or below those of
+the two-half-step V-cycle, which stopped at half the tolerance."""
+import numpy as np
+import pytest
+
+from mhdproj import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(mhdproj, torch, c, **kw):
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    pr = mhdproj.PressureProjection(c["dims"], c["h"], outlet=c["outlet"], **kw)
+    pr.set_coefficients(t(c["alpha"]), t(c["solid"]), c["rho_liquid"], c["rho_air"])
+    return pr, [t(c[k]) for k in "uvw"]
+
+
+def _flat(torch, arrays):
+    return torch.cat([a.double().reshape(-1) for a in arrays])
+
+
+def _rel(a, b):
+    return float((a - b).norm() / b.norm())
+
+
+# relative L2 errors of pressure and velocities with two half-steps
+FORWARD = {"fp16": (8.9e-8, 4.7e-7), "bf16": (1.4e-6, 6.8e-7), "fp32": (7.7e-8, 4.6e-7)}
+
+
+def test_projection_errors_at_full_size(gpu):
+    import mhdproj
+
+    torch = gpu
+    c = synth.make_case("jet256")
+
+    def solve(precision, tol):
+        pr, us = _context(mhdproj, torch, c, precision=precision, rel_tol=tol)
+        u, p, _ = pr.project(us, c["dt"])
+        out = p.double().clone(), _flat(torch, u)
+        pr.close()
+        return out
+
+    exact = solve("fp32", 1e-11)
+    for precision, bound in FORWARD.items():
+        got = solve(precision, 1e-6)
+        for e, b in zip((_rel(g, x) for g, x in zip(got, exact)), bound):
+            assert e <= b, (precision, e, b)
+
+
+ADJOINT = {"fp16": (5.5e-7, 3.7e-7, 5.2e-7), "bf16": (8.1e-7, 5.1e-7, 4.3e-6), "fp32": (5.7e-7, 5.6e-7, 2.9e-6)}
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("precision", ["fp16", "bf16", "fp32"])
+def test_adjoint_errors(gpu, precision, seed):
+    import mhdproj
+
+    torch = gpu
+    c = synth.make_case("jet128", seed=seed)
+    gp = (np.random.default_rng(seed).standard_normal(c["alpha"].shape) * 1e-6 * (c["solid"] == 0)).astype(np.float32)
+    g = []
+    for tol in (1e-6, 1e-11):
+        pr, us = _context(mhdproj, torch, c, precision=precision, rel_tol=tol, gauge=0)
+        g.append(_flat(torch, pr.vjp(us, torch.from_numpy(gp).cuda(), 1e-5)[0]))
+        pr.close()
+    assert _rel(*g) <= ADJOINT[precision][seed - 1]
+
+
+@pytest.mark.parametrize("precision", ["fp16", "bf16", "fp32"])
+def test_slow_flow_to_the_tightest_tolerance(gpu, precision):
+    """A pass aims at a share of the tolerance, but not below what FP32 sums of
+    squares hold: velocities of 1e-5 m/s to 1e-12 are residuals of 1e-21."""
+    import mhdproj
+
+    torch = gpu
+    c = synth.make_case("jet128", scale=0.5)
+    pr, us = _context(mhdproj, torch, c, precision=precision, rel_tol=1e-12)
+    fast, p, st = pr.project(us, c["dt"])
+    fast, p = [v.clone() for v in fast], p.clone()
+    k = 2.0 ** -14
+    slow, ps, ss = pr.project([v * k for v in us], c["dt"])
+    pr.close()
+    assert st.true_relative_residual <= 1e-12 and ss.true_relative_residual <= 1e-12
+    # both within the tolerance of one answer, scaled by a power of two
+    assert _rel(_flat(torch, slow) / k, _flat(torch, fast)) < 1e-7
+    assert _rel(ps.double() / k, p.double()) < 1e-7
