@@ -1834,6 +1834,9 @@ extern "C" int mhdproj_profile_kernels(mhdproj_ctx* ctx, int reps, mhdproj_kerne
     // Algorithmic bytes per cell: the compulsory traffic of each kernel's
     // fields, every field touched once per launch.
     const double vbc = ctx->opt.precision == 0 ? 4.0 : 2.0;   // level-1 vector bytes per cell
+    // The pre-smoothed correction between the two passes: the black half, or
+    // every cell where the passes run two half-steps.
+    const double eb = ctx->pipelined && ctx->mg.lv[0].passes == PASS_PAIR ? 4.0 : 2.0;
     // Connected-component labelling of the solid mask, by kernel: run starts
     // (solid 1 -> label 4), links (solid 1), roots and classes (solid 1 ->
     // class 1); with an outlet the top marks (clear 1).  Labels other than
@@ -1856,10 +1859,10 @@ extern "C" int mhdproj_profile_kernels(mhdproj_ctx* ctx, int reps, mhdproj_kerne
     const Item pipelined[] = {
         // z 4 + p_old 4 + coef 16 + x 4 -> p 4 + x 4 + q 4
         {"search_spmv", 40.0, 1, 10},
-        // r 4 + q 4 + coef -> r 4 + e 4 + coarse r (1/8 cell)
-        {"presmooth_restrict", 16.0 + cb + vbc / 8.0, 1, 11},
-        // e 4 + coarse e (1/8 cell) + r 4 + coef -> z 4
-        {"prolong_postsmooth", 12.0 + cb + vbc / 8.0, 1, 12},
+        // r 4 + q 4 + coef -> r 4 + e + coarse r (1/8 cell)
+        {"presmooth_restrict", 12.0 + eb + cb + vbc / 8.0, 1, 11},
+        // e + coarse e (1/8 cell) + r 4 + coef -> z 4
+        {"prolong_postsmooth", 8.0 + eb + cb + vbc / 8.0, 1, 12},
         // b 8 + x 8 (double-FP32 pairs) + coef 16 -> r 4 + e 4
         {"refinement_residual", 40.0, 0, 7},
         {"coefficients", 29.0, 0, 8},

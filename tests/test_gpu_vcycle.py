@@ -166,3 +166,26 @@ def test_v_cycle_equals_the_fp64_restatement(gpu, dims, periodic, precision):
         got, ref = (np.where(solid == 0, v - v[solid == 0].mean(), 0.0) for v in (got, ref))
     eps = {"fp32": 2.0 ** -24, "fp16": 2.0 ** -12, "bf16": 2.0 ** -9}[precision]
     assert np.abs(got - ref).max() <= 160 * eps * np.abs(ref).max()
+
+
+# whole runs, TMA passes, passes of two half-steps (the correction of every cell)
+@pytest.mark.parametrize("precision,dims,e", [("fp16", (64, 64, 64), 2), ("fp16", (128, 128, 128), 2), ("fp32", (128, 64, 128), 4)])
+def test_profiled_bytes_of_the_passes(gpu, precision, dims, e):
+    """The smoothing passes' compulsory bytes per cell: FP32 r, q and z, the
+    correction as it is stored between them, records, an eighth of a coarse
+    vector value."""
+    import mhdproj
+
+    torch = gpu
+    shape = dims[::-1]
+    pr = mhdproj.PressureProjection(dims, 1e-4, outlet=True, precision=precision)
+    pr.set_coefficients(torch.ones(shape, device="cuda"), torch.zeros(shape, dtype=torch.uint8, device="cuda"), 6440.0, 6440.0)
+    u = [torch.zeros(s, device="cuda") for s in ((shape[0], shape[1], shape[2] + 1), (shape[0], shape[1] + 1, shape[2]),
+                                                 (shape[0] + 1, shape[1], shape[2]))]
+    u[2][:, 0, 0] = 1.0
+    pr.project(u, 1e-5)
+    got = {k["name"]: k["bytes"] for k in pr.profile_kernels()}
+    pr.close()
+    n, records, coarse = dims[0] * dims[1] * dims[2], {"fp32": 16, "fp16": 8}[precision], {"fp32": 4, "fp16": 2}[precision] / 8
+    assert got["presmooth_restrict"] == n * (4 + 4 + records + 4 + e + coarse)
+    assert got["prolong_postsmooth"] == n * (e + coarse + 4 + records + 4)
