@@ -559,9 +559,9 @@ __global__ void __launch_bounds__(kBlock) k_em_initial_reduce(EmDev D) {
 // reductions inside the passes, by the block that arrives last, cost more than
 // their launches (operator 44, residual 31).
 constexpr int kEdges = 4;
-// From here on kEdges edges a thread, one below: two blocks per SM of the long
-// form (28x28x23, 61 thousand edges, 57 blocks of it: 998 us a step against 926).
-constexpr uint32_t kManyEdges = 2u * 152u * kEdges * kBlock;
+// kEdges edges a thread from two blocks per SM of that form on, one below
+// (28x28x23, 61 thousand edges, 57 blocks of it: 998 us a step against 926).
+static bool many_edges(uint32_t edges, int sms) { return edges >= 2u * (uint32_t)sms * kEdges * kBlock; }
 // final_reduce over one or two sums per group, the same order.
 __device__ __forceinline__ void clear(float& v) { v = 0.0f; }
 __device__ __forceinline__ void clear(float2& v) { v = make_float2(0.0f, 0.0f); }
@@ -1224,6 +1224,7 @@ struct mhdproj_em_ctx {
     uint32_t batch_initial = 0;       // the step constants the batch graph was captured with
     uint32_t batch_nodal = 0;
     float batch_dt = 0.0f;
+    int sms = 152;                    // multiprocessors of the context's device
     bool materials = false;
     double time_s = 0.0, last_dt = 0.0;
     bool can_predict = false;
@@ -1332,7 +1333,7 @@ static void em_iteration_n(mhdproj_em_ctx* ctx) {
     ctx->launches += 2;
 }
 static void em_iteration(mhdproj_em_ctx* ctx) {
-    if (ctx->D.E >= kManyEdges) em_iteration_n<kEdges>(ctx);
+    if (many_edges(ctx->D.E, ctx->sms)) em_iteration_n<kEdges>(ctx);
     else em_iteration_n<1>(ctx);
 }
 // The iteration kernels take EmDev by value, so the graph holds the step
@@ -1440,6 +1441,10 @@ int mhdproj_em_create(const mhdproj_em_config* cfg, mhdproj_em_ctx** out) {
         delete ctx;
         return MHDPROJ_ERR_CUDA;
     }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        (void)cudaGetLastError();  // the size rule keeps its default
     ctx->own_stream = true;
     const size_t E = D.E, C = D.cells;
     const size_t groups = std::max(em_groups(D.E), em_groups(D.cells));
