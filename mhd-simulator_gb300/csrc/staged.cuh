@@ -9,11 +9,6 @@ namespace staged {
 
 // cp.async with zero fill: `valid` false copies nothing and writes zeros,
 // which is the value of a cell outside a closed boundary.
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem, bool valid) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    const int n = valid ? 4 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
-}
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     const int n = valid ? 8 : 0;
@@ -23,13 +18,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     const int n = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
-}
-// Copy of two consecutive cells of a vector field (8 bytes FP32, 4 bytes
-// FP16/BF16).
-template <class VT>
-__device__ __forceinline__ void cp_async_pair(void* smem, const VT* gmem, bool valid) {
-    if (sizeof(VT) == 4) cp_async8(smem, gmem, valid);
-    else cp_async4(smem, gmem, valid);
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -75,28 +63,6 @@ constexpr bool axis_wrap_in_range() {
     return true;
 }
 static_assert(axis_wrap_in_range(), "a wrapped coordinate leaves the grid");
-
-// Rotating slot indices of the plane rings: index of plane zA + k.
-struct Slots {
-    int j3, j4, j5;
-    __device__ __forceinline__ Slots() : j3(0), j4(0), j5(0) {}
-    __device__ __forceinline__ void next() {
-        j3 = j3 == 2 ? 0 : j3 + 1;
-        j4 = (j4 + 1) & 3;
-        j5 = j5 == 4 ? 0 : j5 + 1;
-    }
-    __device__ __forceinline__ int s3(int k) const {  // k in -2 .. 2
-        int v = j3 + k;
-        v = v < 0 ? v + 3 : v;
-        return v >= 3 ? v - 3 : v;
-    }
-    __device__ __forceinline__ int s4(int k) const { return (j4 + k) & 3; }
-    __device__ __forceinline__ int s5(int k) const {  // k in -4 .. 4
-        int v = j5 + k;
-        v = v < 0 ? v + 5 : v;
-        return v >= 5 ? v - 5 : v;
-    }
-};
 
 }  // namespace staged
 }  // namespace mhdproj
