@@ -1047,12 +1047,17 @@ void mg_plan_bottom(MGPlan& P) {
     // the inner cycle B converges on that level, which the weight-2 coarse
     // correction does not guarantee; the solver falls back to V-cycles
     // (w_disabled) when CG breaks down.
-    // With the three-half-step passes the second visit (25 us) saves about a
-    // quarter of the iterations, which pays only where the rest of an
-    // iteration takes longer than 100 us: from 48 MB of finest-level records
-    // on (FP16 jet 256^3: 8.2 ms with it, 9.6 without; 256x128x128: 3.6 and
-    // 3.4; 128^3: 2.7 and 2.6; 96^3: 2.0 and 1.9).  The other paths take it
-    // everywhere (w_min_bytes 0).
+    // In the fused passes the second visit (25 us) saves a quarter of the
+    // iterations, which pays where the rest of an iteration takes long: from
+    // 48 MB of finest-level records on.  A projection of a jet without and with
+    // it, us: FP16 128^3 2626 3359, 256x128x128 3275 3358, 160^3 3616 3467, 192^3
+    // 4587 4115, 256^3 8143 7690; BF16 128^3 2476 3514, 256x128x128 3703 4172,
+    // 192^3 4601 4227, 256^3 10437 9525; FP32, whose large levels run two
+    // half-steps, 64^3 1715 2099, 96^3 2353 2552, 128^3 3550 3626, 256x128x64 3600
+    // 3633, 160^3 5132 5088, 192^3 6400 6115.  Between 1.2 and 4 million cells
+    // single grids differ by 10 % either way (FP32 128x128x96 3333 3060, a column
+    // of 256x128x64 2370 2694).  Periodic axes: equal within 7 %.  The per-level
+    // kernels take it everywhere (w_min_bytes 0).
     P.w_from = P.w_to = 0;
     const long long record = P.precision == 0 ? 16 : 8;
     const bool w_pays = P.lv[0].L.g.n() * record >= P.w_min_bytes;
