@@ -310,7 +310,7 @@ static int build_levels(mhdproj_ctx* ctx) {
                     P.lv[l].passes = PASS_RUN;
                 else if (P.precision == 0 && pair_level_init(gl, P.lv[l].sm, P.lv[l].e))
                     P.lv[l].passes = PASS_PAIR;
-                else if (P.precision != 0 && tma_level_init(P.precision, gl, P.lv[l].sm))
+                else if (P.precision != 0 && tma_level_init(gl, P.lv[l].sm))
                     P.lv[l].passes = PASS_TMA;
                 else
                     P.lv[l].passes = PASS_ASYNC;

@@ -210,6 +210,21 @@ __device__ __forceinline__ void finish_rz(double rz_thread, Scalars* sc, double*
     }
 }
 
+// Quad of thread t in a stage over `rows` staged rows from row0 on, and whether
+// there is one: the 16 interior quads of a row go to one half-warp, so its
+// shared-memory accesses are contiguous; the two halo quads of each row follow.
+__device__ __forceinline__ bool stage_task(int t, int rows, int row0, int* row, int* q) {
+    if (t < rows * 16) {
+        *row = row0 + (t >> 4);
+        *q = 1 + (t & 15);
+    } else {
+        const int k = t - rows * 16;
+        *row = row0 + (k >> 1);
+        *q = (k & 1) ? NQ - 1 : 0;
+    }
+    return t < rows * NQ;
+}
+
 template <int N>
 using Phase = std::integral_constant<int, N>;
 

@@ -603,16 +603,18 @@ int f_sms = 0;
 int f_occ[12] = {};
 enum { O_PRE_F32 = 0, O_PRE_LO, O_PRE_LO_UPD, O_PRE_F32_UPD, O_PRE_COARSE, O_POST_F32, O_POST_LO, O_POST_COARSE };
 
-// Even z runs chosen so the grid fills whole waves of resident blocks; each
-// run also computes three planes below and above it and drains one step.  On levels too small to
-// fill one wave the score favours the shortest runs (fewest steps per block).
-Launch fused_launch(const Grid3& g0, int occ_kind, int fty) {
+Launch fused_launch(const Grid3& g, int occ_kind, int fty) {
+    return run_launch(g, dim3(QX, fty, 1), fty, (f_sms > 0 ? f_sms : 152) * (f_occ[occ_kind] > 0 ? f_occ[occ_kind] : 1),
+                      7);
+}
+}  // namespace
+
+Launch run_launch(const Grid3& g, dim3 block, int tile_rows, int cap, int extra) {
     Launch P;
-    P.g = g0;
-    P.block = dim3(QX, fty, 1);
-    const int gx = (g0.nx + PX - 1) / PX, gy = (g0.ny + fty - 1) / fty, nz = g0.nz;
+    P.g = g;
+    P.block = block;
+    const int gx = (g.nx + PX - 1) / PX, gy = (g.ny + tile_rows - 1) / tile_rows, nz = g.nz;
     const int tiles = gx * gy;
-    const int cap = (f_sms > 0 ? f_sms : 152) * (f_occ[occ_kind] > 0 ? f_occ[occ_kind] : 1);
     int best_zper = nz + (nz & 1), best_zc = 1;
     double best = -1.0;
     for (int zc = 1; zc <= nz; zc++) {
@@ -623,7 +625,7 @@ Launch fused_launch(const Grid3& g0, int occ_kind, int fty) {
         const long long blocks = (long long)tiles * zcr;
         if (blocks > MAX_REDUCE_BLOCKS) break;
         const double waves = (double)blocks / cap;
-        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 7));
+        const double score = waves / std::ceil(waves) * ((double)zper / (zper + extra));
         if (score > best) {
             best = score;
             best_zper = zper;
@@ -635,7 +637,6 @@ Launch fused_launch(const Grid3& g0, int occ_kind, int fty) {
     P.nblocks = tiles * best_zc;
     return P;
 }
-}  // namespace
 
 bool fused_supported(const Grid3& g) {
     if (g.nx % 4) return false;

@@ -181,6 +181,11 @@ void launch_search_spmv(const Launch& L, const float4* coef, const float* z, con
 void launch_accumulate_pipelined(const Launch& L, float* x_hi, float* x_lo, const float* x, const float* p0,
                                  const float* p1, const Scalars* sc, cudaStream_t s);
 cudaError_t mg_prepare_attributes();
+// Launch of a pass that marches tiles of 64 x tile_rows columns along z: even
+// runs so chosen that the grid fills whole waves of `cap` resident blocks, each
+// run computing `extra` planes besides its own.  On levels too small to fill one
+// wave the shortest runs win (fewest steps per block).
+Launch run_launch(const Grid3& g, dim3 block, int tile_rows, int cap, int extra);
 // The two passes of a level without periodic axes whose x extent divides by
 // four, records staged by TMA (tma_fused.cu).  Such a level keeps its records
 // in their own layout (tma_records) and its pre-smoothed correction as the
@@ -189,7 +194,7 @@ cudaError_t mg_prepare_attributes();
 cudaError_t tma_prepare_attributes();
 bool tma_level_ok(const Grid3& g);
 size_t tma_record_bytes(const Grid3& g);
-bool tma_level_init(int ck, const Grid3& g, const void* sm);  // tma_level_ok and the copy map encodes
+bool tma_level_init(const Grid3& g, const void* sm);  // tma_level_ok and the copy map encodes
 void tma_records(int ck, const Launch& L, const void* coef, void* sm, cudaStream_t s);
 void tma_level_residual(int ck, const Launch& L, const void* sm, const void* r, const void* e, void* r2,
                         const Scalars* sc, cudaStream_t s);

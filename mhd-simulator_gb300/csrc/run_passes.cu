@@ -43,21 +43,6 @@ struct RunSm {
     float2 zpart[2][WTY][QX];
 };
 
-// Quad of thread t in a stage over `rows` staged rows from row0 on: the 16
-// interior quads of a row go to one half-warp, so its shared-memory accesses
-// are contiguous; the two halo quads of each row follow.
-__device__ __forceinline__ bool stage_task(int t, int rows, int row0, int* row, int* q) {
-    if (t < rows * 16) {
-        *row = row0 + (t >> 4);
-        *q = 1 + (t & 15);
-    } else {
-        const int k = t - rows * 16;
-        *row = row0 + (k >> 1);
-        *q = (k & 1) ? NQ - 1 : 0;
-    }
-    return t < rows * NQ;
-}
-
 // All planes' records, zero outside the grid.
 template <int CK>
 __device__ __forceinline__ void stage_records(RunSm<CK>& S, const typename CoefStore<CK>::T* sm, const Grid3& g, int x0,

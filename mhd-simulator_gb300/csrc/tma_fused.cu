@@ -58,7 +58,6 @@
 // a timeout), and finishes its loop without waiting again.  Periodic grids
 // (a copy box cannot wrap around) take the passes of fused_kernels.cu.
 #include <algorithm>
-#include <cmath>
 #include <cstdlib>
 
 #include "kernels.h"
@@ -77,7 +76,6 @@ constexpr int NO = 10;         // octets of a staged row: x0-8 .. x0+71
 constexpr int QO = PX / 8;     // own octets of a row
 constexpr int RS = 4 * HH;     // entries of a staged record row
 
-template <int CK>
 struct OGeo {
     static constexpr int FTY = 32;                     // tile rows
     static constexpr int RH = FTY + 6;                 // staged rows y0-3 .. y0+FTY+2
@@ -115,10 +113,9 @@ __device__ __forceinline__ void rec_hi(const Rec4<CK>& r, float (&o)[4]) {
     o[0] = half_hi<CK>(r.v.x); o[1] = half_hi<CK>(r.v.y); o[2] = half_hi<CK>(r.v.z); o[3] = half_hi<CK>(r.v.w);
 }
 
-template <int CK>
 struct PassSm {
     using ET = Entry;
-    using G = OGeo<CK>;
+    using G = OGeo;
     alignas(128) ET c[G::NS][G::RH][RS];
     // the three stages' half-planes, each for the next step (slot: step & 1)
     alignas(16) float ex[3][2][G::RH][HH];
@@ -254,10 +251,9 @@ __device__ __forceinline__ void block_bar() { asm volatile("bar.sync 0;\n" ::: "
 
 // The plane ring of records: issue, wait and slot bookkeeping shared by the
 // two passes.
-template <int CK>
 struct RecordRing {
-    using G = OGeo<CK>;
-    using SM = PassSm<CK>;
+    using G = OGeo;
+    using SM = PassSm;
     static constexpr int ISSUER = G::NT - 1;
     static constexpr unsigned BYTES = G::RH * RS * sizeof(Entry);
     SM& S;
@@ -340,14 +336,14 @@ static_assert(rc_exchange_ordered(), "a slot of restriction sums is overwritten 
 // formed first, written for the tile's cells, and ||r_out||^2 decides
 // convergence.  FINE: the right-hand side is sigma * r.
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
-__global__ void __launch_bounds__(OGeo<CK>::NT, 1)
+__global__ void __launch_bounds__(OGeo::NT, 1)
     k_pre_tma(const __grid_constant__ CUtensorMap tm_rec, Grid3 g, Grid3 gc, const VT* __restrict__ rin,
               const float* __restrict__ q, float* __restrict__ r_out, VT* __restrict__ ek, VTc* __restrict__ rc,
               Scalars* sc, double* partials, int nblocks) {
     if (sc->converged) return;
     using ET = Entry;
-    using G = OGeo<CK>;
-    using SM = PassSm<CK>;
+    using G = OGeo;
+    using SM = PassSm;
     using R4 = typename Raw4<VT>::T;
     constexpr int NT = G::NT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -387,7 +383,7 @@ __global__ void __launch_bounds__(OGeo<CK>::NT, 1)
         }
     };
     load(zs);
-    RecordRing<CK> ring(S, &tm_rec, x0, y0, zs);
+    RecordRing ring(S, &tm_rec, x0, y0, zs);
     float rr_thread = 0.f;
     // restriction sums of the coarse planes of planes k-3 and k-1; the finished
     // ones of the even rows until the odd rows' arrive
@@ -526,15 +522,15 @@ __global__ void __launch_bounds__(OGeo<CK>::NT, 1)
 // (VT).  DOT (finest level): r . out / sigma gives rz and beta; the next
 // V-cycle's sigma is then taken from ||r||^2.
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
-__global__ void __launch_bounds__(OGeo<CK>::NT, 1)
+__global__ void __launch_bounds__(OGeo::NT, 1)
     k_post_tma(const __grid_constant__ CUtensorMap tm_rec, Grid3 g, Grid3 gc, const VT* __restrict__ ek,
                const VTc* __restrict__ ec, const VT* __restrict__ rin, VT* __restrict__ out,
                const VT* __restrict__ accum, float w, Scalars* sc, double* partials, int nblocks,
                long long n_active) {
     if (sc->converged) return;
     using ET = Entry;
-    using G = OGeo<CK>;
-    using SM = PassSm<CK>;
+    using G = OGeo;
+    using SM = PassSm;
     using R4 = typename Raw4<VT>::T;
     using P2 = typename Raw2<VT>::T;
     using C2 = typename Raw2<VTc>::T;
@@ -578,7 +574,7 @@ __global__ void __launch_bounds__(OGeo<CK>::NT, 1)
         }
     };
     load(zs);
-    RecordRing<CK> ring(S, &tm_rec, x0, y0, zs);
+    RecordRing ring(S, &tm_rec, x0, y0, zs);
     Acc acc_rz;
     // the octet's values by step parity: prolonged blacks (index 1-H: plane k-1,
     // H: k-2), first reds (H: k-2, 1-H: k-3), changes of the blacks (1-H: k-3,
@@ -783,7 +779,7 @@ int g_occ[3][2][2] = {};  // [records precision][coarse level][down / up]: resid
 
 // 4-D map of the records: (entries of a half row, four half rows, y, z), box
 // HH x 4 x rows x 1; entries beyond nx/2 are out of bounds (zero).
-bool rec_map(CUtensorMap* m, const void* base, int ck, const Grid3& g, int rows) {
+bool rec_map(CUtensorMap* m, const void* base, const Grid3& g, int rows) {
     const cuuint64_t es = 4;
     const cuuint64_t half = (cuuint64_t)rec_pitch(g.nx) * es;
     const cuuint64_t dims[4] = {(cuuint64_t)(g.nx / 2), 4, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
@@ -796,56 +792,26 @@ bool rec_map(CUtensorMap* m, const void* base, int ck, const Grid3& g, int rows)
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Even z runs that fill whole waves of resident blocks; each run computes
-// three planes below and above it.
-Launch tma_launch(const Grid3& g0, int fty, int nt, int occ) {
-    Launch P;
-    P.g = g0;
-    P.block = dim3(nt, 1, 1);
-    const int gx = (g0.nx + PX - 1) / PX, gy = (g0.ny + fty - 1) / fty, nz = g0.nz;
-    const int tiles = gx * gy;
-    const int cap = (g_sms > 0 ? g_sms : 152) * (occ > 0 ? occ : 1);
-    int best_zper = nz + (nz & 1), best_zc = 1;
-    double best = -1.0;
-    for (int zc = 1; zc <= nz; zc++) {
-        int zper = (nz + zc - 1) / zc;
-        if (zper & 1) zper++;
-        if (zper < 2 && zc > 1) break;
-        const int zcr = (nz + zper - 1) / zper;
-        const long long blocks = (long long)tiles * zcr;
-        if (blocks > MAX_REDUCE_BLOCKS) break;
-        const double waves = (double)blocks / cap;
-        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 6));
-        if (score > best) {
-            best = score;
-            best_zper = zper;
-            best_zc = zcr;
-        }
-    }
-    P.grid = dim3(gx, gy, best_zc);
-    P.g.zper = best_zper;
-    P.nblocks = tiles * best_zc;
-    return P;
+Launch tma_launch(const Grid3& g, int occ) {
+    return run_launch(g, dim3(OGeo::NT, 1, 1), OGeo::FTY, (g_sms > 0 ? g_sms : 152) * (occ > 0 ? occ : 1), 6);
 }
 
 template <int CK, class VT, class VTc, bool UPDATE, bool FINE>
 void pre_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q, float* r_out, void* e,
              void* rc, Scalars* sc, double* partials, cudaStream_t s) {
-    using G = OGeo<CK>;
     CUtensorMap tm_rec;
-    (void)rec_map(&tm_rec, sm, CK, g, G::RH);  // the same encode succeeded at tma_level_init
-    const Launch P = tma_launch(g, G::FTY, G::NT, g_occ[CK][FINE ? 0 : 1][0]);
-    k_pre_tma<CK, VT, VTc, UPDATE, FINE><<<P.grid, P.block, sizeof(PassSm<CK>) + 128, s>>>(
+    (void)rec_map(&tm_rec, sm, g, OGeo::RH);  // the same encode succeeded at tma_level_init
+    const Launch P = tma_launch(g, g_occ[CK][FINE ? 0 : 1][0]);
+    k_pre_tma<CK, VT, VTc, UPDATE, FINE><<<P.grid, P.block, sizeof(PassSm) + 128, s>>>(
         tm_rec, P.g, gc, (const VT*)rin, q, r_out, (VT*)e, (VTc*)rc, sc, partials, P.nblocks);
 }
 template <int CK, class VT, class VTc, bool DOT, bool FINE>
 void post_tma(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r, void* out,
               const void* accum, float w, Scalars* sc, double* partials, long long n_active, cudaStream_t s) {
-    using G = OGeo<CK>;
     CUtensorMap tm_rec;
-    (void)rec_map(&tm_rec, sm, CK, g, G::RH);  // the same encode succeeded at tma_level_init
-    const Launch P = tma_launch(g, G::FTY, G::NT, g_occ[CK][FINE ? 0 : 1][1]);
-    k_post_tma<CK, VT, VTc, DOT, FINE><<<P.grid, P.block, sizeof(PassSm<CK>) + 128, s>>>(
+    (void)rec_map(&tm_rec, sm, g, OGeo::RH);  // the same encode succeeded at tma_level_init
+    const Launch P = tma_launch(g, g_occ[CK][FINE ? 0 : 1][1]);
+    k_post_tma<CK, VT, VTc, DOT, FINE><<<P.grid, P.block, sizeof(PassSm) + 128, s>>>(
         tm_rec, P.g, gc, (const VT*)e, (const VTc*)ec, (const VT*)r, (VT*)out, (const VT*)accum, w, sc, partials,
         P.nblocks, n_active);
 }
@@ -858,9 +824,9 @@ cudaError_t prep(F* fn, size_t bytes, int threads, int* occ) {
 }
 template <int CK, class VT, class VTc>
 cudaError_t prep_level(bool fine) {
-    using G = OGeo<CK>;
+    using G = OGeo;
     cudaError_t e = cudaSuccess;
-    const size_t bytes = sizeof(PassSm<CK>) + 128;
+    const size_t bytes = sizeof(PassSm) + 128;
     if (fine) {
         if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, true, true>, bytes, G::NT, &g_occ[CK][0][0]);
         if (e == cudaSuccess) e = prep(k_pre_tma<CK, VT, VTc, false, true>, bytes, G::NT, nullptr);
@@ -901,9 +867,9 @@ cudaError_t tma_prepare_attributes() {
 }
 
 bool tma_level_ok(const Grid3& g) { return g_tma_enabled && g.periodic == 0 && g.nx % 4 == 0; }
-bool tma_level_init(int ck, const Grid3& g, const void* sm) {
+bool tma_level_init(const Grid3& g, const void* sm) {
     CUtensorMap tm;
-    return tma_level_ok(g) && rec_map(&tm, sm, ck, g, OGeo<1>::RH);
+    return tma_level_ok(g) && rec_map(&tm, sm, g, OGeo::RH);
 }
 size_t tma_record_bytes(const Grid3& g) { return (size_t)g.ny * g.nz * 4 * rec_pitch(g.nx) * sizeof(Entry); }
 void tma_records(int ck, const Launch& L, const void* coef, void* sm, cudaStream_t s) {

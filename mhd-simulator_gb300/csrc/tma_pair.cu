@@ -30,7 +30,6 @@
 // issuing copies, marks the solve as stalled and converged (the host reports a
 // timeout), and finishes its loop without waiting again.
 #include <algorithm>
-#include <cmath>
 
 #include "kernels.h"
 #include "fused_common.cuh"
@@ -81,21 +80,6 @@ struct PairPostSm {
     unsigned long long bar[2];
     int abort_;
 };
-// Task of thread t in a stage over `rows` staged rows starting at row0: the
-// 16 interior quads (1 .. 16) of a row go to one half-warp, so its
-// shared-memory accesses are contiguous and free of bank conflicts; the two
-// halo quads of each row (0 and 17) follow as tasks rows*16 .. rows*18-1.
-__device__ __forceinline__ void stage_task(int t, int rows, int row0, int* row, int* q) {
-    if (t < rows * 16) {
-        *row = row0 + (t >> 4);
-        *q = 1 + (t & 15);
-    } else {
-        const int e = t - rows * 16;
-        *row = row0 + (e >> 1);
-        *q = (e & 1) ? NQ - 1 : 0;
-    }
-}
-
 }  // namespace
 
 // ------------------------------------------------------ pre-smoothing pass
@@ -148,8 +132,7 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
 
     // red task
     int r_row, r_q;
-    stage_task(t, RH, 0, &r_row, &r_q);
-    const bool has_red = t < G::NRED;
+    const bool has_red = stage_task(t, RH, 0, &r_row, &r_q);
     const int r_o = r_row * RW + 2 * r_q;             // split offset of the quad's even half
     const int r_v = r_row * VW + 4 * r_q;  // its cells in a copied vector row
     const int r_qv = r_row * VW + 4 * r_q;
@@ -160,8 +143,7 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
                           : -1;
     // black task
     int b_row, b_q;
-    stage_task(t, G::NBR, 1, &b_row, &b_q);
-    const bool has_blk = t < G::NBLK;
+    const bool has_blk = stage_task(t, G::NBR, 1, &b_row, &b_q);
     const int b_o = b_row * RW + 2 * b_q;
     const int b_par = (y0 - 2 + b_row) & 1;
     // tile task: the own quad
@@ -334,8 +316,7 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
     if (t == ISSUER) issue(0, 0);
 
     int r_row, r_q;
-    stage_task(t, RH, 0, &r_row, &r_q);
-    const bool has_red = t < G::NRED;
+    const bool has_red = stage_task(t, RH, 0, &r_row, &r_q);
     const int r_o = r_row * RW + 2 * r_q;
     const int r_v = r_row * VW + 4 * r_q;
     const int r_gx = x0 - XO + 4 * r_q, r_gy = y0 - 2 + r_row;
@@ -350,8 +331,7 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
     };
     parents(zs);
     int b_row, b_q;
-    stage_task(t, G::NBR, 1, &b_row, &b_q);
-    const bool has_blk = t < G::NBLK;
+    const bool has_blk = stage_task(t, G::NBR, 1, &b_row, &b_q);
     const int b_o = b_row * RW + 2 * b_q;
     const int b_par = (y0 - 2 + b_row) & 1;
     const bool has_own = t < G::NOWN;
@@ -494,38 +474,9 @@ bool rec_map(CUtensorMap* m, const void* base, const Grid3& g, int rows) {
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// z runs as in fused_launch: even runs that fill whole waves of resident
-// blocks, each run computing two planes below and above it.
-Launch pair_launch(const Grid3& g0, int occ) {
-    Launch P;
-    P.g = g0;
-    P.block = dim3(PGeo::NT, 1, 1);
-    const int gx = (g0.nx + PX - 1) / PX, gy = (g0.ny + PGeo::FTY - 1) / PGeo::FTY, nz = g0.nz;
-    const int tiles = gx * gy;
-    const int cap = (p_sms > 0 ? p_sms : 152) * (occ > 0 ? occ : 1);
-    int best_zper = nz + (nz & 1), best_zc = 1;
-    double best = -1.0;
-    for (int zc = 1; zc <= nz; zc++) {
-        int zper = (nz + zc - 1) / zc;
-        if (zper & 1) zper++;
-        if (zper < 2 && zc > 1) break;
-        const int zcr = (nz + zper - 1) / zper;
-        const long long blocks = (long long)tiles * zcr;
-        if (blocks > MAX_REDUCE_BLOCKS) break;
-        const double waves = (double)blocks / cap;
-        const double score = waves / std::ceil(waves) * ((double)zper / (zper + 4));
-        if (score > best) {
-            best = score;
-            best_zper = zper;
-            best_zc = zcr;
-        }
-    }
-    P.grid = dim3(gx, gy, best_zc);
-    P.g.zper = best_zper;
-    P.nblocks = tiles * best_zc;
-    return P;
+Launch pair_launch(const Grid3& g, int occ) {
+    return run_launch(g, dim3(PGeo::NT, 1, 1), PGeo::FTY, (p_sms > 0 ? p_sms : 152) * (occ > 0 ? occ : 1), 4);
 }
-
 
 template <bool UPDATE, bool FINE>
 void pre_pair(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, const float* q, float* r_out, void* e,
