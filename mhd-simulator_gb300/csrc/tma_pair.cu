@@ -54,6 +54,7 @@ struct PGeo {
     static_assert(NBLK <= NT && NOWN <= NT && NRED < NT, "one task per thread");
 };
 constexpr int VW = RW;  // staged rows of a level vector: x0-4 .. x0+67
+constexpr int CVW = 44, CVH = PGeo::RH / 2;  // staged coarse rows: x0/2-8 .. x0/2+35, y0/2-1 .. y0/2+4
 
 // Shared memory of the pre-smoothing pass: records and corrections of planes
 // zA-3 .. zA+1 (five slots), the copied residual and q of planes zA, zA+1.
@@ -70,9 +71,11 @@ struct PairPreSm {
 };
 // Shared memory of the post-smoothing pass: records and smoothed corrections
 // of planes zA-3 .. zA+1, the copied pre-smoothed correction and right-hand
-// side of planes zA, zA+1.
+// side of planes zA, zA+1, and (COPY) the coarse planes of two pairs of planes.
+template <bool COPY>
 struct PairPostSm {
     using G = PGeo;
+    alignas(128) float ec[COPY ? 2 : 1][COPY ? (CVH * CVW + 31) / 32 * 32 : 32];
     alignas(128) float4 c[G::NS][G::RH][RW];
     alignas(128) float ev[2][G::RH][VW];
     alignas(128) float rv[2][G::RH][VW];
@@ -271,17 +274,19 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
 }
 
 // ----------------------------------------------------- post-smoothing pass
-// e and r arrive through tm_e and tm_r, the records through tm_rec.  Step structure as in
-// k_pre_pair.
-template <bool FINE>
+// e and r arrive through tm_e and tm_r, the records through tm_rec, the coarse
+// correction through tm_c (COPY) or by a load per quad, where coarse rows are
+// no whole 16 bytes (x extents that 8 does not divide).  256^3: 141 us a pass with
+// the copies, 152 with the loads.  Step structure as in k_pre_pair.
+template <bool FINE, bool COPY>
 __global__ void __launch_bounds__(PGeo::NT, 2)
     k_post_pair(const __grid_constant__ CUtensorMap tm_rec, const __grid_constant__ CUtensorMap tm_e,
-               const __grid_constant__ CUtensorMap tm_r, Grid3 g, Grid3 gc, const float* __restrict__ ec,
-               float* __restrict__ out, const float* __restrict__ accum, float w, Scalars* sc, double* partials,
+               const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_c, Grid3 g, Grid3 gc,
+               const float* __restrict__ ec, float* __restrict__ out, const float* __restrict__ accum, float w, Scalars* sc, double* partials,
                int nblocks, long long n_active) {
     if (sc->converged) return;
     using G = PGeo;
-    using SM = PairPostSm;
+    using SM = PairPostSm<COPY>;
     constexpr int FTY = G::FTY, NT = G::NT, RH = G::RH, NS = G::NS, SL = RH * RW;
     constexpr unsigned BYTES = RH * RW * sizeof(float4) + 2 * RH * VW * sizeof(float);
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -300,10 +305,12 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
         const int zz = zs + k;
         unsigned long long* b = &S.bar[k & 1];
         fence_proxy_async();
-        mbar_expect_tx(b, BYTES);
+        mbar_expect_tx(b, BYTES + (COPY && !(k & 1) ? CVH * CVW * (unsigned)sizeof(float) : 0u));
         tma_4d(&S.c[0][0][0] + off, &tm_rec, 2 * x0 - 8, 0, y0 - 2, zz, b);
         tma_3d(&S.ev[k & 1][0][0], &tm_e, x0 - XO, y0 - 2, zz, b);
         tma_3d(&S.rv[k & 1][0][0], &tm_r, x0 - XO, y0 - 2, zz, b);
+        // zs is even: an even step starts a coarse plane
+        if (COPY && !(k & 1)) tma_3d(&S.ec[(k >> 1) & 1][0], &tm_c, (x0 >> 1) - 8, (y0 >> 1) - 1, zz >> 1, b);
         last_issued = k;
     };
     if (t == ISSUER) {
@@ -322,14 +329,16 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
     const int r_gx = x0 - XO + 4 * r_q, r_gy = y0 - 2 + r_row;
     const int r_par = r_gy & 1;
     const bool r_inside = has_red && r_gx >= 0 && r_gx < g.nx && r_gy >= 0 && r_gy < g.ny;
-    // the quad's two coarse parents, loaded one plane ahead (their rows need no
-    // alignment here, which a copy would)
+    // the quad's two coarse parents: their place in the copied plane, or loaded two
+    // steps before the pair of planes that shares them (168 us one step ahead and
+    // on every plane)
+    const int r_ce = (r_row >> 1) * CVW + 6 + 2 * r_q;
     const long long r_c = r_inside ? (r_gx >> 1) + (long long)gc.nx * (r_gy >> 1) : 0, csxy = (long long)gc.nx * gc.ny;
-    float2 cnext = make_float2(0.f, 0.f);
-    auto parents = [&](int zz) {
+    float2 ccur = make_float2(0.f, 0.f), cnext = ccur;
+    auto parents = [&](int zz) {  // of planes zz and zz + 1, zz even
         cnext = ldg_pair<float>(ec + r_c + csxy * (zz >> 1), r_inside && zz >= 0 && zz < g.nz);
     };
-    parents(zs);
+    if (!COPY) parents(zs);
     int b_row, b_q;
     const bool has_blk = stage_task(t, G::NBR, 1, &b_row, &b_q);
     const int b_o = b_row * RW + 2 * b_q;
@@ -362,13 +371,17 @@ __global__ void __launch_bounds__(PGeo::NT, 2)
         if (has_red) {
             float* EP = e0 + o0;
             float4 ev = make_float4(0.f, 0.f, 0.f, 0.f), rq = ev;
-            const float2 cv = cnext;
+            float2 cv = make_float2(0.f, 0.f);
+            if (!COPY && !(P & 1)) {
+                ccur = cnext;
+                parents(zA + 2);
+            }
             if (r_inside && zA >= 0 && zA < g.nz) {
+                cv = COPY ? *reinterpret_cast<const float2*>(&S.ec[P >> 1][0] + r_ce) : ccur;
                 ev = cvt4r<float>(*reinterpret_cast<const float4*>(&S.ev[P & 1][0][0] + r_v));
                 rq = cvt4r<float>(*reinterpret_cast<const float4*>(&S.rv[P & 1][0][0] + r_v));
             }
             const int p = r_par ^ (P & 1);
-            parents(zA + 1);
             const float2 er = p ? make_float2(ev.y, ev.w) : make_float2(ev.x, ev.z);
             const float2 rb = p ? make_float2(rq.x, rq.z) : make_float2(rq.y, rq.w);
             *reinterpret_cast<float2*>(EP + r_o + p * HW) = make_float2(fmaf(w, cv.x, er.x), fmaf(w, cv.y, er.y));
@@ -449,11 +462,11 @@ namespace {
 // ------------------------------------------------------------------ host
 int p_sms = 0, p_occ[2][2] = {};  // [fine 0, coarse 1][pre, post]
 
-// 3-D map of a level vector (x-fastest cells), box VW x rows x 1.
-bool vec_map(CUtensorMap* m, const void* base, const Grid3& g, int rows) {
+// 3-D map of a level vector (x-fastest cells), box of width x rows x 1.
+bool vec_map(CUtensorMap* m, const void* base, const Grid3& g, int rows, int width = VW) {
     const cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
     const cuuint64_t strides[2] = {(cuuint64_t)g.nx * 4, (cuuint64_t)g.nx * g.ny * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)VW, (cuuint32_t)rows, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)width, (cuuint32_t)rows, 1};
     const cuuint32_t es[3] = {1, 1, 1};
     return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                     const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -489,17 +502,18 @@ void pre_pair(const Grid3& g, const Grid3& gc, const void* sm, const void* rin, 
     k_pre_pair<UPDATE, FINE><<<P.grid, P.block, sizeof(PairPreSm<UPDATE>) + 128, s>>>(
         tm_rec, tm_r, tm_q, P.g, gc, r_out, (float*)e, (float*)rc, sc, partials, P.nblocks);
 }
-template <bool FINE>
-void post_pair(const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r, void* out,
-               const void* accum, float w, Scalars* sc, double* partials, long long n_active, cudaStream_t s) {
+template <bool FINE, bool COPY>
+void post_pair(const CUtensorMap& tm_c, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec,
+               const void* r, void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active,
+               cudaStream_t s) {
     CUtensorMap tm_rec, tm_e, tm_r;
     (void)rec_map(&tm_rec, sm, g, PGeo::RH);
     (void)vec_map(&tm_e, e, g, PGeo::RH);
     (void)vec_map(&tm_r, r, g, PGeo::RH);
     const Launch P = pair_launch(g, p_occ[FINE ? 0 : 1][1]);
-    k_post_pair<FINE><<<P.grid, P.block, sizeof(PairPostSm) + 128, s>>>(
-        tm_rec, tm_e, tm_r, P.g, gc, (const float*)ec, (float*)out, (const float*)accum, w, sc, partials, P.nblocks,
-        n_active);
+    k_post_pair<FINE, COPY><<<P.grid, P.block, sizeof(PairPostSm<COPY>) + 128, s>>>(
+        tm_rec, tm_e, tm_r, tm_c, P.g, gc, (const float*)ec, (float*)out, (const float*)accum, w, sc, partials,
+        P.nblocks, n_active);
 }
 cudaError_t prep(const void* fn, size_t bytes, int* occ) {
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -514,9 +528,11 @@ cudaError_t pair_prepare_attributes() {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = prep((const void*)k_pre_pair<true, true>, sizeof(PairPreSm<true>) + 128, &p_occ[0][0]);
     if (e == cudaSuccess) e = prep((const void*)k_pre_pair<false, true>, sizeof(PairPreSm<false>) + 128, nullptr);
-    if (e == cudaSuccess) e = prep((const void*)k_post_pair<true>, sizeof(PairPostSm) + 128, &p_occ[0][1]);
+    if (e == cudaSuccess) e = prep((const void*)k_post_pair<true, true>, sizeof(PairPostSm<true>) + 128, &p_occ[0][1]);
+    if (e == cudaSuccess) e = prep((const void*)k_post_pair<true, false>, sizeof(PairPostSm<false>) + 128, nullptr);
     if (e == cudaSuccess) e = prep((const void*)k_pre_pair<false, false>, sizeof(PairPreSm<false>) + 128, &p_occ[1][0]);
-    if (e == cudaSuccess) e = prep((const void*)k_post_pair<false>, sizeof(PairPostSm) + 128, &p_occ[1][1]);
+    if (e == cudaSuccess) e = prep((const void*)k_post_pair<false, true>, sizeof(PairPostSm<true>) + 128, &p_occ[1][1]);
+    if (e == cudaSuccess) e = prep((const void*)k_post_pair<false, false>, sizeof(PairPostSm<false>) + 128, nullptr);
     return e;
 }
 // A level of FP32 records whose rows the copies can read: no periodic axis, nx
@@ -533,8 +549,12 @@ void pair_pre(bool fine, bool update, const Grid3& g, const Grid3& gc, const voi
 }
 void pair_post(bool fine, const Grid3& g, const Grid3& gc, const void* sm, const void* e, const void* ec, const void* r,
                void* out, const void* accum, float w, Scalars* sc, double* partials, long long n_active, cudaStream_t s) {
-    if (fine) post_pair<true>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
-    else post_pair<false>(g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s);
+    CUtensorMap tm_c = {};  // read where coarse rows are whole 16 bytes
+    const bool copy = gc.nx % 4 == 0 && vec_map(&tm_c, ec, gc, CVH, CVW);
+#define POST(FINE, COPY) post_pair<FINE, COPY>(tm_c, g, gc, sm, e, ec, r, out, accum, w, sc, partials, n_active, s)
+    if (copy) fine ? POST(true, true) : POST(false, true);
+    else fine ? POST(true, false) : POST(false, false);
+#undef POST
 }
 
 }  // namespace mhdproj
