@@ -860,10 +860,15 @@ static void begin_scalars(mhdproj_ctx* ctx, bool adjoint = false) {
     // the restart forgets the search space.  Relative L2 errors of the pressure
     // at 1e-6 off a solve to 1e-11, jet 256^3 FP16 / BF16 / FP32 (and ms):
     //   two half-steps, half the tolerance     8.9e-8 1.4e-6 7.7e-8 (11.3 11.4 14.0)
-    //   first pass 1e-5, aim 1/16              3.0e-7 2.0e-6 -      ( 8.5  9.2 -)
+    //   first pass 1e-5, aim 1/16 (FP32 1/2)   3.0e-7 2.0e-6 1.3e-7 ( 8.5  9.2 14.3)
     //   first pass 1e-5, aim 1/32 (FP32 1/8)   3.0e-7 8.0e-9 9.4e-8 ( 9.1 12.9 15.5)
-    //   first pass 4.9e-6, aim 1/32 (FP32 1/8) 8.7e-8 1.7e-8 5.0e-8 ( 8.7 12.0 14.9)
-    // 4.9e-6 is half of the smallest tolerance that a single pass serves.
+    //   first pass 4.9e-6, aim 1/32 (FP32 1/8) 8.7e-8 1.7e-8 5.0e-8 ( 8.7 12.0 14.4)
+    // 4.9e-6 is half of the smallest tolerance that a single pass serves.  Below
+    // 1e-6 the passes aim at 1/64: at 1e-8 FP16 256^3 that is 4.4e-8 off FP64, the
+    // rounding of an FP32 pressure, in 13.1 ms, 9.4e-8 in 10.0 with 1/32 and 7.0e-8
+    // in 13.4 with two half-steps; at 1e-6 it changes no error but costs an
+    // iteration (eight solves of a chain at 128^3 and their adjoints: 40.5 ms, 44.1
+    // with 1/64).
     // An adjoint's right-hand side has more weight on smooth modes, and its goal
     // lies close to the reduction that a pass stops at: its first pass runs on to
     // 1e-7.  vjp jet 128^3 BF16, three seeds: 8.1e-7 5.1e-7 4.3e-6 with two
@@ -873,7 +878,8 @@ static void begin_scalars(mhdproj_ctx* ctx, bool adjoint = false) {
     const MGPlan& P = ctx->mg;
     PassGoals goals = {1.0 / 4, 1e-10, 1.0};
     if (ctx->pipelined)
-        goals = {P.lv[0].passes == PASS_PAIR ? 1.0 / 64 : 1.0 / 1024, adjoint ? 1e-14 : 2.4e-11, 1.0 / 16};
+        goals = {P.lv[0].passes == PASS_PAIR ? 1.0 / 64 : (ctx->opt.rel_tol < 9e-7f ? 1.0 / 4096 : 1.0 / 1024),
+                 adjoint ? 1e-14 : 2.4e-11, 1.0 / 16};
     launch_init_scalars(ctx->sc, tol2, abs_floor, goals, (int)ctx->opt.max_iterations, ctx->stream);
 }
 
