@@ -12,8 +12,8 @@
 //   red, black (over-relaxed), red half-steps       z        = the smoothed correction
 //   [fine level] r . z for the CG step length.
 // Three half-steps instead of two (red and black down, black and red up) cut
-// the CG iterations by a third to a half (column 160x120x96, periodic y: 12 ->
-// 8 at a quarter of the stopping residual).
+// the CG iterations by a quarter to a half (column 160x120x96, periodic x and y, at
+// 1e-6: 12 -> 9).
 // Both march a 64 x 32 (x, y) tile along z (64 x 16 with FP32 records).  The
 // stages of one pass run as a pipeline over planes: in one step the
 // pre-smoothing pass forms the residual and the first red values of plane z,

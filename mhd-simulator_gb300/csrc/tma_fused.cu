@@ -13,8 +13,8 @@
 //                     e_r = (r + sum beta e_b)/d
 // The up pass is the down pass reversed, so the cycle is symmetric.  Against
 // one red and one black half-step per pass the third one cuts the CG
-// iterations (jet 256^3: 22 -> 13, column 512x256x256: 14 -> 7, at an eighth of
-// the stopping residual) while the HBM traffic of a pass stays the same.  After
+// iterations (jet 256^3: 23 -> 15, column 512x256x256: 13 -> 7, at 1e-6 and smaller
+// errors) while the HBM traffic of a pass stays the same.  After
 // the down pass the residual is zero on red cells, so the restriction sums
 // black residuals only; the up pass overwrites the red values first, so only
 // the black half of the down pass's correction is kept in HBM (compact rows of
@@ -37,14 +37,15 @@
 //    the z-high mobilities of the next stage: they pass on in registers;
 //  * the steps of the two parities are straight-line code, one copy for the
 //    warps with the tile's octets and one for the halo's.
-// What bounds it: the latency of a step (about 2200 cycles: the stages' shared
-// memory loads and dependent sums, twelve warps per SM) and the L2 traffic of
-// the halo (1.5 reads per cell).  jet 256^3, FP16 records: 121 us down, 120 us
-// up (400 and 335 MB of HBM traffic).  Passes of two half-steps on quads with
-// every neighbour from shared memory took 101 and 98 us; three half-steps in
-// that form would take half as long again.  16 tile rows and two blocks per
-// SM: 142 and 154 us (halo 1.7, registers capped at 128); values of earlier
-// planes from shared memory instead of registers: 152 and 192 us.
+// What bounds it: the latency of a step (about 2700 cycles down and 3100 up, the
+// stages' shared memory loads and dependent sums, twelve warps per SM, issue
+// slots busy 0.39 and 0.36 of the time) and the L2 traffic of the halo (1.5 reads
+// per cell).  jet 256^3, FP16 records: 106 us down, 121 us up (403 and 333 MB of
+// HBM traffic).  Passes of two half-steps on quads with every neighbour from
+// shared memory took 101 and 98 us; three half-steps in that form would take
+// half as long again.  16 tile rows and two blocks per SM: 142 and 154 us (halo
+// 1.7, registers capped at 128); values of earlier planes from shared memory
+// instead of registers: 152 and 192 us.
 //
 // Records in HBM: per grid row four half rows of `pitch` entries: (beta_x,
 // beta_y) of the even-x cells, of the odd-x cells, (beta_z, diagonal) of the
