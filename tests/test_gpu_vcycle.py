@@ -189,3 +189,11 @@ def test_profiled_bytes_of_the_passes(gpu, precision, dims, e):
     n, records, coarse = dims[0] * dims[1] * dims[2], {"fp32": 16, "fp16": 8}[precision], {"fp32": 4, "fp16": 2}[precision] / 8
     assert got["presmooth_restrict"] == n * (4 + 4 + records + 4 + e + coarse)
     assert got["prolong_postsmooth"] == n * (e + coarse + 4 + records + 4)
+
+
+@pytest.mark.parametrize("dims", [(24, 16, 160), (28, 16, 160), (24, 72, 35), (136, 9, 75)], ids=str)
+def test_fp32_pair_passes_on_narrow_and_ragged_grids(gpu, dims):
+    """The FP32 passes of two half-steps, their coarse rows copied (x extents
+    that 8 divides) or loaded: coarse planes smaller than a copy's box, rows and
+    planes that end inside a pair."""
+    test_v_cycle_equals_the_fp64_restatement(gpu, dims, 0, "fp32")
