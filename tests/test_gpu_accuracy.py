@@ -1,7 +1,8 @@
 """Errors of solves at their tolerance.  The stopping rules look at the norm of
 the residual, which says little about an isolated smooth mode, so the errors
 themselves are held: against a solve to 1e-11 they stay at or below those of
-the two-half-step V-cycle, which stopped at half the tolerance."""
+the two-half-step V-cycle, which stopped at half the tolerance (SLACK: the
+build may round otherwise)."""
 import numpy as np
 import pytest
 
